@@ -19,10 +19,10 @@
 // cleared at the start of every call, and calls that overlap on the GPU (on
 // different streams, or from different host threads) race on it.
 //
-// The sweep is one thread per row, summing the row in CSR order with the
-// reference's float operations (src/pr/omp_base.cc:34-39), so its scores are
-// identical to the reference's; the residual is reduced in FP64 per CTA and
-// combined by the last CTA of each sweep.
+// The sweep sums each row in CSR order with the reference's float operations
+// (src/pr/omp_base.cc:34-39), so its scores are identical to the reference's;
+// the residual is reduced in FP64 per CTA and combined by the last CTA of each
+// sweep.
 #include <math.h>
 #include <string.h>
 
@@ -37,6 +37,9 @@ namespace {
 constexpr int kNoAllocMaxVertices = 1 << 20;  // largest m accepted
 constexpr int kNoAllocMaxIter = 1000;         // largest max_iter accepted
 constexpr int kNoAllocBlock = 256;
+// Edges a CTA stages in shared memory at a time: 16 independent loads per
+// thread, 16 KB per CTA (8 CTAs per SM stay resident).
+constexpr int kNoAllocTile = 16 * kNoAllocBlock;
 constexpr int kNoAllocMaxCtas = (kNoAllocMaxVertices + kNoAllocBlock - 1) / kNoAllocBlock;
 
 // Byte layout of the scratch array (all offsets 256-byte aligned).
@@ -91,9 +94,19 @@ __global__ void k_na_prologue(NoAllocArgs a) {
 
 // One sweep; sweep index and done flag live in the scratch words, so launches
 // after convergence return at once.
+//
+// A CTA owns 256 consecutive rows, whose edges are one contiguous range: all
+// threads stage the range's contributions tile by tile in shared memory
+// (coalesced indices, 16 gathers in flight per thread), and each thread then
+// adds its own row's part in CSR order.  What bounds a sweep is the longest
+// row's chain of dependent adds; with one thread per row loading its own edges
+// that chain held an L2 round trip per few edges (RMAT, 250,007 vertices, edge
+// factor 16: 820 us per sweep, 0.06 instructions issued per cycle; the call
+// with 24 sweeps 16.9 ms, staged 2.6 ms).
 __global__ void __launch_bounds__(kNoAllocBlock) k_na_sweep(NoAllocArgs a) {
   __shared__ int s_it, s_last;
   __shared__ double red[kNoAllocBlock / 32];
+  __shared__ float s_val[kNoAllocTile];
   if (threadIdx.x == 0) {
     const int done = *(volatile int *)(a.words + 2);
     s_it = done ? -1 : *(volatile int *)(a.words + 1);
@@ -103,15 +116,38 @@ __global__ void __launch_bounds__(kNoAllocBlock) k_na_sweep(NoAllocArgs a) {
   if (it < 0) return;
   const float *cin = (it & 1) ? a.c1 : a.c0;
   float *cout = (it & 1) ? a.c0 : a.c1;
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r0 = blockIdx.x * kNoAllocBlock, v = r0 + threadIdx.x;
+  const bool has = v < a.m;
+  const int first = a.rowptr[r0], end = a.rowptr[min(a.m, r0 + kNoAllocBlock)];
+  const int e0 = has ? a.rowptr[v] : end, e1 = has ? a.rowptr[v + 1] : end;
+  const float so = has ? a.s[v] : 0.f;
+  const int od = has ? a.outdeg[v] : 1;
+  float total = 0.f;
+  for (long long t = first; t < end; t += kNoAllocTile) {
+    const int n = (int)min((long long)kNoAllocTile, end - t);
+    int c[kNoAllocTile / kNoAllocBlock];
+#pragma unroll
+    for (int q = 0; q < kNoAllocTile / kNoAllocBlock; ++q) {
+      const int i = q * kNoAllocBlock + threadIdx.x;
+      c[q] = i < n ? a.col[t + i] : -1;
+    }
+    float x[kNoAllocTile / kNoAllocBlock];
+#pragma unroll
+    for (int q = 0; q < kNoAllocTile / kNoAllocBlock; ++q) x[q] = c[q] >= 0 ? cin[c[q]] : 0.f;
+    __syncthreads();  // the previous tile has been added
+#pragma unroll
+    for (int q = 0; q < kNoAllocTile / kNoAllocBlock; ++q)
+      s_val[q * kNoAllocBlock + threadIdx.x] = x[q];
+    __syncthreads();
+    const int lo = (int)max(0LL, e0 - t), hi = (int)min((long long)n, e1 - t);
+#pragma unroll 8
+    for (int i = lo; i < hi; ++i) total = __fadd_rn(total, s_val[i]);
+  }
   double err = 0.0;
-  if (v < a.m) {
-    float total = 0.f;
-    for (int e = a.rowptr[v]; e < a.rowptr[v + 1]; ++e) total = __fadd_rn(total, cin[a.col[e]]);
-    const float so = a.s[v];
+  if (has) {
     const float sn = __fadd_rn(a.base, __fmul_rn(a.damp, total));
     a.s[v] = sn;
-    cout[v] = __fdiv_rn(sn, __int2float_rn(a.outdeg[v]));
+    cout[v] = __fdiv_rn(sn, __int2float_rn(od));
     err = (double)fabsf(__fsub_rn(sn, so));
   }
   err = warp_sum_d(err);

@@ -88,3 +88,25 @@ def test_noalloc_rejects_sizes_beyond_its_scratch(G):
     with pytest.raises(G.GprError) as e:
         G.pagerank_noalloc(limit + 1, 0, 1, 1, 1, 1)
     assert e.value.status == G.GPR_EINVAL and "limit" in str(e.value)
+
+
+@pytest.mark.parametrize("hub,deg", [(0, 1), (255, 4095), (256, 4096), (300, 4097), (9999, 9998)])
+def test_noalloc_long_rows_at_tile_edges(G, O, hub, deg):
+    """A row as long as the staged tile, one edge shorter and longer, and longer
+    than two tiles, at the first, last and an inner row of a CTA: every score
+    equals the oracle's bit for bit (the same float additions in CSR order)."""
+    torch = pytest.importorskip("torch")
+    from graphs import in_csr
+    rng = np.random.default_rng(hub + deg)
+    m = 10000
+    src = rng.choice(np.delete(np.arange(m), hub), deg, replace=False)
+    more = rng.integers(0, m, (2, 3 * m))
+    more = more[:, more[1] != hub]
+    rp, col, od = in_csr(m, np.concatenate([src, more[0]]),
+                         np.concatenate([np.full(deg, hub), more[1]]))
+    assert rp[hub + 1] - rp[hub] == deg
+    d_rp, d_col, d_od = (torch.from_numpy(a).cuda() for a in (rp, col, od))
+    d_s = torch.full((m,), float(np.float32(1.0) / np.float32(m)), device="cuda")
+    G.pagerank_noalloc(m, len(col), d_rp, d_col, d_od, d_s, tol=0.0, max_iter=4)
+    ref, _, _ = O.pr_plain_f32(rp, col, od, tol=0.0, max_iter=4)
+    assert np.array_equal(d_s.cpu().numpy(), ref)
