@@ -38,7 +38,7 @@ constexpr int kNoAllocMaxVertices = 1 << 20;  // largest m accepted
 constexpr int kNoAllocMaxIter = 1000;         // largest max_iter accepted
 constexpr int kNoAllocBlock = 256;
 // Edges a CTA stages in shared memory at a time: 16 independent loads per
-// thread, 16 KB per CTA (8 CTAs per SM stay resident).
+// thread.  Half of that measured slower: a long row pays for every tile's end.
 constexpr int kNoAllocTile = 16 * kNoAllocBlock;
 constexpr int kNoAllocMaxCtas = (kNoAllocMaxVertices + kNoAllocBlock - 1) / kNoAllocBlock;
 
@@ -92,18 +92,102 @@ __global__ void k_na_prologue(NoAllocArgs a) {
   if (i < a.m) a.c0[i] = __fdiv_rn(a.s[i], __int2float_rn(a.outdeg[i]));
 }
 
+// acc + v[lo] + ... + v[hi - 1] in order.  The loads of a batch are issued before
+// its additions, so a value costs an addition's latency and not a load's as well
+// (about 6 cycles against 33).
+__device__ __forceinline__ float add_in_order(const float *v, int lo, int hi, float acc) {
+  for (; lo < hi; lo += 16) {
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = lo + i < hi ? v[lo + i] : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (lo + i < hi) acc = __fadd_rn(acc, x[i]);
+  }
+  return acc;
+}
+
+// Values of a long row per lane and step of ordered_sum; odd, so that the
+// lanes' strides fall on different shared-memory banks.
+constexpr int kOrdV = 31;
+// Rows with more values than this in a staged tile are added by their warp.
+// One thread adds at about 6 cycles a value; the warp's step costs 450 cycles
+// for up to 992 values, and a row starts with one or two sequential stretches.
+constexpr int kOrdMin = 384;
+
+// acc + v[lo] + v[lo + 1] + ... + v[hi - 1], each addition rounded to nearest
+// even as __fadd_rn does in that order, by one warp (all lanes call it with
+// the same arguments and get the sum).
+//
+// While the running sum stays within one binade it is A * u for an integer A in
+// [2^23, 2^24), and adding x >= 0 rounds x / u to an integer by itself: only
+// where x / u lies halfway between two integers does the result depend on A
+// (on its parity).  So where no value is halfway and the sum stays in the
+// binade, the roundings are independent, the integers can be added in any order,
+// and their total is added to the sum's bits.  Each lane takes kOrdV
+// consecutive values (x / u = y, an exact scaling by a power of two; y < 2^22, so
+// that adding 1.5 * 2^23 rounds y to the nearest integer and leaves it in the
+// low bits).  Lanes before the first one that meets a halfway value, a y out of
+// range (a negative, infinite or NaN value among them) or the end of the binade
+// are accepted; that lane's values are added one by one, and the next step
+// starts behind them with the new binade.  A step that accepts few lanes adds
+// a longer stretch one by one.
+__device__ float ordered_sum(const float *v, int lo, int hi, float acc, int lane) {
+  constexpr float kRound = 12582912.f;  // 1.5 * 2^23
+  constexpr unsigned kRoundBits = 0x4B400000u, kTooBig = 0x4A800000u;  // 2^22
+  while (lo < hi) {
+    const unsigned bits = __float_as_uint(acc), eb = bits >> 23;
+    int take = 0;  // lanes accepted
+    if (eb >= 23u && eb < 255u) {  // positive, finite, and 2^s below is a normal float
+      const float scale = __uint_as_float((277u - eb) << 23);
+      const int b = lo + lane * kOrdV;
+      unsigned sum = 0u, top = 0u;
+      bool half = false;
+#pragma unroll
+      for (int q = 0; q < kOrdV; ++q) {
+        const float y = b + q < hi ? __fmul_rn(v[b + q], scale) : 0.f;
+        const float t = __fadd_rn(y, kRound);
+        half |= fabsf(__fsub_rn(y, __fsub_rn(t, kRound))) == 0.5f;
+        sum += __float_as_uint(t) - kRoundBits;
+        top = max(top, __float_as_uint(y));
+      }
+      const bool bad = half || top >= kTooBig;
+      const unsigned room = 0x7FFFFFu - (bits & 0x7FFFFFu);  // largest total that stays
+      if (bad || sum > room) sum = room + 1u;
+      // sums of lanes up to each; room + 1 <= 2^23 a lane, so nothing wraps
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += t;
+      }
+      const unsigned stop = __ballot_sync(0xffffffffu, sum > room);
+      take = stop ? __ffs(stop) - 1 : 32;
+      const unsigned total = __shfl_sync(0xffffffffu, sum, max(take, 1) - 1);
+      if (take > 0) acc = __uint_as_float(bits + total);
+      lo = min(hi, lo + take * kOrdV);
+    }
+    if (take < 32) {
+      const int e = min(hi, lo + (take < 4 ? 2 : 1) * kOrdV);
+      acc = add_in_order(v, lo, e, acc);
+      lo = e;
+    }
+  }
+  return acc;
+}
+
 // One sweep; sweep index and done flag live in the scratch words, so launches
 // after convergence return at once.
 //
 // A CTA owns 256 consecutive rows, whose edges are one contiguous range: all
 // threads stage the range's contributions tile by tile in shared memory
 // (coalesced indices, 16 gathers in flight per thread), and each thread then
-// adds its own row's part in CSR order.  What bounds a sweep is the longest
-// row's chain of dependent adds; with one thread per row loading its own edges
-// that chain held an L2 round trip per few edges (RMAT, 250,007 vertices, edge
-// factor 16: 820 us per sweep, 0.06 instructions issued per cycle; the call
-// with 24 sweeps 16.9 ms, staged 2.6 ms).
-__global__ void __launch_bounds__(kNoAllocBlock) k_na_sweep(NoAllocArgs a) {
+// adds its own row's part in CSR order; long parts are added by the row's warp
+// (ordered_sum).  What bounds a sweep is the longest row's chain of dependent
+// adds.  RMAT, 250,007 vertices, edge factor 16, 24 sweeps: with one thread per
+// row loading its own edges the chain held an L2 round trip per few edges (820 us
+// per sweep, 0.06 instructions issued per cycle, 16.9 ms per call); staged, and
+// one thread adding a row, 2.6 ms per call; with ordered_sum 1.4 ms.
+__global__ void __launch_bounds__(kNoAllocBlock, 6) k_na_sweep(NoAllocArgs a) {
   __shared__ int s_it, s_last;
   __shared__ double red[kNoAllocBlock / 32];
   __shared__ float s_val[kNoAllocTile];
@@ -123,25 +207,33 @@ __global__ void __launch_bounds__(kNoAllocBlock) k_na_sweep(NoAllocArgs a) {
   const float so = has ? a.s[v] : 0.f;
   const int od = has ? a.outdeg[v] : 1;
   float total = 0.f;
+  constexpr int kPer = kNoAllocTile / kNoAllocBlock;
   for (long long t = first; t < end; t += kNoAllocTile) {
     const int n = (int)min((long long)kNoAllocTile, end - t);
-    int c[kNoAllocTile / kNoAllocBlock];
+    int c[kPer];
 #pragma unroll
-    for (int q = 0; q < kNoAllocTile / kNoAllocBlock; ++q) {
+    for (int q = 0; q < kPer; ++q) {
       const int i = q * kNoAllocBlock + threadIdx.x;
       c[q] = i < n ? a.col[t + i] : -1;
     }
-    float x[kNoAllocTile / kNoAllocBlock];
+    float x[kPer];
 #pragma unroll
-    for (int q = 0; q < kNoAllocTile / kNoAllocBlock; ++q) x[q] = c[q] >= 0 ? cin[c[q]] : 0.f;
+    for (int q = 0; q < kPer; ++q) x[q] = c[q] >= 0 ? cin[c[q]] : 0.f;
     __syncthreads();  // the previous tile has been added
 #pragma unroll
-    for (int q = 0; q < kNoAllocTile / kNoAllocBlock; ++q)
-      s_val[q * kNoAllocBlock + threadIdx.x] = x[q];
+    for (int q = 0; q < kPer; ++q) s_val[q * kNoAllocBlock + threadIdx.x] = x[q];
     __syncthreads();
     const int lo = (int)max(0LL, e0 - t), hi = (int)min((long long)n, e1 - t);
-#pragma unroll 8
-    for (int i = lo; i < hi; ++i) total = __fadd_rn(total, s_val[i]);
+    unsigned longs = __ballot_sync(0xffffffffu, hi - lo > kOrdMin);
+    if (hi - lo <= kOrdMin) total = add_in_order(s_val, lo, hi, total);
+    __syncwarp();
+    for (; longs; longs &= longs - 1) {
+      const int src = __ffs(longs) - 1;
+      const float sum = ordered_sum(s_val, __shfl_sync(0xffffffffu, lo, src),
+                                    __shfl_sync(0xffffffffu, hi, src),
+                                    __shfl_sync(0xffffffffu, total, src), threadIdx.x & 31);
+      if ((threadIdx.x & 31) == src) total = sum;
+    }
   }
   double err = 0.0;
   if (has) {

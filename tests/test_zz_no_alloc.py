@@ -110,3 +110,41 @@ def test_noalloc_long_rows_at_tile_edges(G, O, hub, deg):
     G.pagerank_noalloc(m, len(col), d_rp, d_col, d_od, d_s, tol=0.0, max_iter=4)
     ref, _, _ = O.pr_plain_f32(rp, col, od, tol=0.0, max_iter=4)
     assert np.array_equal(d_s.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "equal", "halves", "zeros", "wide", "tiny", "negative",
+                                  "infinite"])
+def test_noalloc_long_rows_add_in_order(G, O, kind):
+    """Long rows are added by a warp as integers within a binade where that gives
+    what the additions in CSR order give; whatever the values (ties, zeros, sums
+    that leave their binade at once, denormal, negative and infinite ones), the
+    scores are the oracle's bits."""
+    torch = pytest.importorskip("torch")
+    from graphs import in_csr
+    rng = np.random.default_rng(len(kind))
+    m, hubs = 12000, 40
+    counts = rng.integers(200, 9000, hubs)
+    src = np.concatenate([rng.choice(m, n, replace=False) for n in counts]
+                         + [rng.integers(0, m, 4 * m)])
+    dst = np.concatenate([np.repeat(np.arange(hubs) * 7, counts), rng.integers(0, m, 4 * m)])
+    rp, col, od = in_csr(m, src, dst)
+    s0 = rng.random(m).astype(np.float32)
+    if kind == "equal":
+        s0 = np.full(m, 1.0 / m, dtype=np.float32)
+    elif kind == "halves":
+        s0 = (rng.integers(0, 64, m) / 64 * od).astype(np.float32)
+    elif kind == "zeros":
+        s0[rng.random(m) < 0.7] = 0.0
+    elif kind == "wide":
+        s0 = np.exp(rng.normal(0, 18, m)).astype(np.float32)
+    elif kind == "tiny":
+        s0 *= np.float32(1e-38)
+    elif kind == "negative":
+        s0 -= np.float32(0.5)
+    elif kind == "infinite":
+        s0[m // 2] = np.inf
+    d_rp, d_col, d_od = (torch.from_numpy(a).cuda() for a in (rp, col, od))
+    d_s = torch.from_numpy(s0.copy()).cuda()
+    G.pagerank_noalloc(m, len(col), d_rp, d_col, d_od, d_s, tol=0.0, max_iter=3)
+    ref, _, _ = O.pr_plain_f32(rp, col, od, scores=s0, tol=0.0, max_iter=3)
+    assert np.array_equal(d_s.cpu().numpy(), ref, equal_nan=True)
