@@ -260,7 +260,7 @@ struct gpr_graph {
   int hot_bytes = 0;           // shared-memory budget of the hot prefix
   int grid_hot[12] = {0};      // cooperative grid of each persistent sweep kernel
   void *h0 = nullptr, *h1 = nullptr;  // BF16 contributions of the mixed form (on first use)
-  int *wq = nullptr;           // [2] work-queue heads of the hot kernel
+  int *wq = nullptr;           // [2] chunk-queue heads of the blocked form
   bool hot_ok = false;         // every hot-kernel variant is co-resident at grid_hot
   int grid_step = 0, max_grid = 0;
   bool coop = false;

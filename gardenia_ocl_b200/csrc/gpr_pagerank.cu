@@ -63,8 +63,8 @@ struct PrArgs {
   int bar_expect;
   long long timeout_ns;
   int hot;                // contributions [0, hot) are staged in shared memory
-  int *wq;                // [2] work-queue heads of the hot kernel, by sweep parity
-  int batch;              // units per work-queue grab
+  int *wq;                // [2] blocked form: chunk-queue heads by sweep parity
+  int batch;              // blocked form: chunks per work-queue grab
   unsigned long long cond;  // graph mode: while-node condition handle (0: none)
   // blocked form (gpr_blocked.cu): tiles of source-ordered entries per block
   int n_tiles, acc_rows;  // acc_rows: high words of the shared accumulators start here
@@ -236,106 +236,101 @@ __device__ __forceinline__ double block_sum(double v) {
   return t;
 }
 
-// Grid barrier that also reduces the per-CTA residuals of sweep `it` into
-// err_hist[it].  The CTA that arrives last sums the partials in CTA order
-// (deterministic) and opens the next generation.  Every wait is bounded by
-// timeout_ns of %globaltimer; on expiry the CTA raises status[0] bit 0 and
-// the caller returns.  Requires co-resident CTAs (cooperative launch).
-__device__ bool barrier_reduce(const PrArgs &a, int it, double cta_total) {
-  __shared__ int s_state;
-  __shared__ unsigned s_gen;
-  const unsigned G = gridDim.x;
-  if (threadIdx.x == 0) {
-    a.cta_err[(size_t)(it & 1) * G + blockIdx.x] = cta_total;
-    s_gen = ld_acquire(a.bar + 1);
-    __threadfence();
-    const unsigned arrived = atomicAdd(a.bar, 1u);
-    s_state = (arrived == (unsigned)a.bar_expect - 1u) ? 1 : 0;
-  }
-  __syncthreads();
-  if (s_state == 1) {
-    if (threadIdx.x < 32) {
-      __threadfence();
-      const double *src = a.cta_err + (size_t)(it & 1) * G;
-      double t = 0.0;
-      for (unsigned i = threadIdx.x; i < G; i += 32) t += __ldcg(src + i);
-      t = warp_sum(t);
-      if (threadIdx.x == 0) {
-        a.err_hist[it] = t;
-        if (a.wq) atomicExch(a.wq + (it & 1), 0);  // reused by sweep it + 2
-        if (a.tq) atomicExch(a.tq + (it & 1), 0);
-        atomicExch(a.bar, 0u);
-        __threadfence();
-        atomicAdd(a.bar + 1, 1u);
-      }
+// End of sweep `it` in a persistent kernel: this CTA's residual is stored, then
+// the bounded grid barrier (grid_barrier_count; on expiry the caller returns).
+// Behind it CTA 0 resets the queue heads that sweep it + 2 reuses (its arrival
+// at the next barrier orders that before their use).  Requires co-resident
+// CTAs (cooperative launch).
+__device__ __forceinline__ bool close_sweep(const PrArgs &a, int it, double cta_total) {
+  if (threadIdx.x == 0) a.cta_err[(size_t)(it & 1) * gridDim.x + blockIdx.x] = cta_total;
+  if (!grid_barrier_count(a.bar, (unsigned)a.bar_expect * (unsigned)(it + 1), a.status,
+                          a.timeout_ns))
+    return false;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (a.tq) {
+      atomicExch(a.wq + (it & 1), 0);
+      atomicExch(a.tq + (it & 1), 0);
     }
-  } else if (threadIdx.x == 0) {
-    const long long t0 = global_ns();
-    unsigned spins = 0;
-    while (ld_acquire(a.bar + 1) == s_gen) {
-      if ((++spins & 31u) == 0 && global_ns() - t0 > a.timeout_ns) {
-        atomicOr(a.status, 1);
-        s_state = 2;
-        break;
-      }
-      __nanosleep(100);
-    }
-    __threadfence();
   }
-  __syncthreads();
-  return s_state != 2;
+  return true;
+}
+
+// Residual of sweep `it` behind its barrier, by one warp of every CTA: the CTAs'
+// values in a fixed order (the same bits in every CTA), recorded by CTA 0.
+// Each CTA sums for itself, so no CTA waits for one that sums and publishes, and
+// the other warps of the CTA start the next sweep's staging meanwhile.
+__device__ __forceinline__ double sweep_residual(const PrArgs &a, int it, int lane) {
+  const double *src = a.cta_err + (size_t)(it & 1) * gridDim.x;
+  double t = 0.0;
+  for (unsigned i = lane; i < gridDim.x; i += 32) t += __ldcg(src + i);
+  t = warp_sum(t);
+  if (lane == 0 && blockIdx.x == 0) a.err_hist[it] = t;
+  return t;
 }
 
 // All sweeps in one cooperative launch, one 1024-thread CTA per SM.
 // Each sweep first stages contributions [0, hot) -- the vertices of highest
 // in-degree, which a power-law graph gathers most -- into shared memory, so
-// those gathers never reach the L1->L2 request path.  Warps take batches of
-// kQueueBatch chunk/slice units from a global work queue (one head per sweep
-// parity, reset by the barrier); the batch size is chosen so each warp makes
-// about four grabs per sweep, which keeps the single queue head cold while
-// the light units at the end of the queue still balance the tail.
+// those gathers never reach the L1->L2 request path.  The chunk / slice units
+// are in descending size and are dealt out to the CTAs, forward and backward
+// in turn (consecutive units on different SMs); a CTA's warps take its units
+// from a counter in shared memory, the next one while they work on one.  With
+// one global queue the claims of all warps queued on one L2 word and the heavy
+// units, claimed in a burst, fell on few SMs; dealt out to single warps a CTA
+// waited for its slowest warp.  Sweep loop, RMAT, queue / dealt to warps / to CTAs:
+// 250,007 vertices (51 sweeps) 1.17 / 0.87 / 0.78 ms, 1,000,003 (50 sweeps)
+// 2.17 / 1.99 / 1.81 ms, 2^24 (8 sweeps) dealing all 6.16 ms, dealing 85% and
+// queueing the rest 6.10.
 // Zero-in-degree rows are spread over all warps in the two sweeps that need
 // them.
-
 template <int U, int U4, bool GENERIC, int MINB, typename T>
 __global__ void __launch_bounds__(1024, MINB) k_pr_hot(PrArgs a) {
   extern __shared__ float4 s_hot4[];
+  __shared__ double s_total;
+  __shared__ int s_next;
   T *s_hot = reinterpret_cast<T *>(s_hot4);
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
-  const long long gw = (long long)blockIdx.x * nwarps + (threadIdx.x >> 5);
-  const long long nw = (long long)gridDim.x * nwarps;
+  const int gw = warp * gridDim.x + blockIdx.x;
+  const int nw = gridDim.x * nwarps;
   const Policies pol = make_policies();
   const int n_heavy = a.n_chunks + a.n_slices;
+  const int G = gridDim.x, n_mine = (n_heavy + G - 1) / G;
   int it = 0;
-  while (it < a.max_iter) {
+  for (;;) {
     const T *cin = static_cast<const T *>((it & 1) ? a.c1 : a.c0);
     T *cout = static_cast<T *>((it & 1) ? a.c0 : a.c1);
+    // the residual of the sweep before, while the other warps stage
+    if (it > 0 && warp == 0) {
+      const double t = sweep_residual(a, it - 1, lane);
+      if (lane == 0) s_total = t;
+    }
+    if (threadIdx.x == 0) s_next = nwarps;
     const float4 *src = reinterpret_cast<const float4 *>(cin);
     const int n16 = (int)((size_t)a.hot * sizeof(T) / 16);
     for (int i = threadIdx.x; i < n16; i += blockDim.x) s_hot4[i] = ld_contrib4(src + i, pol.keep);
     __syncthreads();
+    if (it > 0 && (it >= a.max_iter || s_total < a.tol)) break;
     using Gat = typename std::conditional<GENERIC, HotGatherGeneric<T>, HotGather<T>>::type;
     const Gat gat{cin, s_hot, a.hot, pol.keep};
     double err = 0.0;
-    for (;;) {
-      int u0 = 0;
-      if (lane == 0) u0 = atomicAdd(a.wq + (it & 1), a.batch);
-      u0 = __shfl_sync(kFull, u0, 0);
-      if (u0 >= n_heavy) break;
-      const int u1 = min(u0 + a.batch, n_heavy);
-      for (int u = u0; u < u1; ++u) {
-        if (u < a.n_chunks) err += do_chunk<U4>(a, gat, cout, u, lane, pol);
-        else err += do_slice<U>(a, gat, cout, u - a.n_chunks, lane, pol);
-      }
+    auto unit = [&](int u) {
+      if (u < a.n_chunks) err += do_chunk<U4>(a, gat, cout, u, lane, pol);
+      else err += do_slice<U>(a, gat, cout, u - a.n_chunks, lane, pol);
+    };
+    // this CTA's dealt units, taken by its warps from a shared counter
+    for (int k = warp; k < n_mine;) {
+      int next = 0;
+      if (lane == 0) next = atomicAdd(&s_next, 1);
+      const int u = k * G + ((k & 1) ? G - 1 - (int)blockIdx.x : (int)blockIdx.x);
+      if (u < n_heavy) unit(u);
+      k = __shfl_sync(kFull, next, 0);
     }
     if (it < 2)
-      for (long long z = gw; z < a.n_zblk; z += nw) err += do_zero(a, cout, (int)z, lane, it, pol);
+      for (int z = gw; z < a.n_zblk; z += nw) err += do_zero(a, cout, z, lane, it, pol);
     const double tot = block_sum(err);
-    if (!barrier_reduce(a, it, tot)) return;
-    const double total = __ldcg(a.err_hist + it);
+    if (!close_sweep(a, it, tot)) return;
     ++it;
-    if (total < a.tol) break;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.status[1] = it;
@@ -357,16 +352,27 @@ template <int PV, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_pr_blocked(PrArgs a) {
   extern __shared__ unsigned s_acc[];  // [2 * acc_rows]: low / high words
   __shared__ int s_tile, s_next_tile, s_last, s_next;
+  __shared__ double s_total;
   const int lane = threadIdx.x & 31;
   const long long gw = (long long)blockIdx.x * (NT / 32) + (threadIdx.x >> 5);
   const long long nw = (long long)gridDim.x * (NT / 32);
   const Policies pol = make_policies();
   int it = 0;
-  while (it < a.max_iter) {
+  for (;;) {
     const float *cin = static_cast<const float *>((it & 1) ? a.c1 : a.c0);
     float *cout = static_cast<float *>((it & 1) ? a.c0 : a.c1);
     double err = 0.0;
-    if (threadIdx.x == 0) s_next_tile = atomicAdd(a.tq + (it & 1), 1);
+    // the first tile's claim and the residual of the sweep before together (a
+    // claim made when the solve is over is never used)
+    if (threadIdx.x == 32) s_next_tile = atomicAdd(a.tq + (it & 1), 1);
+    if (it > 0) {
+      if (threadIdx.x < 32) {
+        const double t = sweep_residual(a, it - 1, lane);
+        if (lane == 0) s_total = t;
+      }
+      __syncthreads();
+      if (it >= a.max_iter || s_total < a.tol) break;
+    }
     for (;;) {
       __syncthreads();
       if (threadIdx.x == 0) s_tile = s_next_tile;
@@ -398,10 +404,8 @@ __global__ void __launch_bounds__(NT, MINB) k_pr_blocked(PrArgs a) {
     if (it < 2)
       for (long long z = gw; z < a.n_zblk; z += nw) err += do_zero(a, cout, (int)z, lane, it, pol);
     const double tot = block_sum(err);
-    if (!barrier_reduce(a, it, tot)) return;
-    const double total = __ldcg(a.err_hist + it);
+    if (!close_sweep(a, it, tot)) return;
     ++it;
-    if (total < a.tol) break;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.status[1] = it;
@@ -592,6 +596,10 @@ const SweepKernels kKernels[] = {
     {(const void *)k_pr_hot<16, 4, true, 1, bf16>, k_pr_step<16, 4, bf16>, 1, 227328, 2},
 };
 constexpr int kHotBlock = 1024;
+// A small graph takes a CTA for every 8 units, up to one per SM: a sweep is then
+// the latency of its units, and fewer of them on an SM are faster (10,007 vertices,
+// 246 units: 32 / 16 / 8 / 4 per CTA 108 / 97 / 94 / 94 us for 13 sweeps).
+constexpr int kUnitsPerCta = 8;
 constexpr int kNumVariants = 8;
 constexpr int kBf16Kernel = 8;
 constexpr int kNumKernels = sizeof(kKernels) / sizeof(kKernels[0]);
@@ -646,11 +654,6 @@ PrArgs make_args(gpr_graph *g, const gpr_pr_opts &o, int ki) {
   a.bar_expect = g->grid_hot[ki];
   a.hot = hot_entries(g, ki);
   a.wq = g->wq;
-  {
-    const long long heavy = (long long)L.n_chunks + L.n_slices;
-    const long long warps = (long long)g->grid_hot[ki] * (kHotBlock / 32);
-    a.batch = (int)std::max<long long>(1, heavy / (warps * 4));
-  }
   a.timeout_ns = (long long)(o.timeout_s * 1e9);
   return a;
 }
@@ -818,7 +821,7 @@ int create_impl(int m, long long nnz, const int *any_rowptr, const int *any_col,
                                                            kHotBlock, smem));
     if (per_sm < kKernels[v].ctas_per_sm) g->hot_ok = false;
     g->grid_hot[v] = (int)std::max<long long>(
-        1, std::min<long long>((long long)sms * kKernels[v].ctas_per_sm, gpr::ceil_div(heavy, 32)));
+        1, std::min<long long>((long long)sms * kKernels[v].ctas_per_sm, gpr::ceil_div(heavy, kUnitsPerCta)));
   }
   GPR_TRY(gpr::dalloc(&g->wq, 2, "work queue"));
   long long step = need < 1 ? 1 : need;

@@ -265,3 +265,18 @@ def test_fp16_form_is_reported_unsupported(G, O):
         with pytest.raises(G.GprError) as e:
             mg.pagerank(precision=G.PREC_FP16)
         assert e.value.status == G.GPR_EUNSUPPORTED
+
+
+@pytest.mark.parametrize("m", [20, 32 * 8, 32 * 9 + 1, 32 * 8 * 148, 32 * 8 * 148 + 33,
+                               32 * 33 * 148 + 5])
+def test_units_dealt_to_ctas(G, O, m):
+    # One unit, a CTA's 8 units and one more, a unit short of and past 8 per SM,
+    # and more units per CTA than it has warps: rows of at most 64 in-edges, so
+    # every score is the reference's bit for bit whatever warp takes a row.
+    rp, col, od = erdos_renyi(m, 8, seed=m)
+    assert np.diff(rp).max() <= 64
+    s, st, hist, _ = solve(G, rp, col, od, tol=0.0, max_iter=5)
+    ref, _, ref_hist = O.pr_plain_f32(rp, col, od, tol=0.0, max_iter=5)
+    assert st.iterations == 5
+    assert np.array_equal(s, ref)
+    np.testing.assert_allclose(hist, ref_hist, rtol=1e-12)
