@@ -297,6 +297,7 @@ struct gpr_graph {
   gpr::BlockedLayout B;
   bool has_blocked = false, blocked_ok = false;
   int grid_blocked = 0, blocked_ctas = 1;  // blocked-form CTAs: total, per SM
+  int blocked_carve = 0;       // shared-memory share of the SM for them, percent
   int *tq = nullptr;
   unsigned *fx_max = nullptr;
   alignas(8) unsigned char loop_args[512] = {0};

@@ -725,6 +725,7 @@ struct gpr_multigraph {
   gpr::BlockedLayout B;
   bool has_blocked = false, blocked_ok = false;
   int grid_blocked = 0, blocked_ctas = 1, max_gm = 0;
+  int blocked_carve = 0;  // shared-memory share of the SM for the blocked kernel, percent
   int *tq = nullptr, *tb = nullptr, *lazy_b = nullptr;
   std::vector<int> lazy_bh;     // graphs with vertices but no tiles
   double *terr = nullptr;
@@ -1082,8 +1083,10 @@ int build_multi(gpr_multigraph *g, const int *h_voff, const int *d_rowptr, const
       GPR_CUDA(cudaFuncGetAttributes(&fa, k));
       const long long need = (long long)g->blocked_ctas * (smem + (long long)fa.sharedSizeBytes + 1024);
       const int carve = (int)std::min<long long>(100, gpr::ceil_div(100 * need, smem_sm));
-      GPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      GPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    8 * gpr::kBlockedMaxRows));
       GPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
+      g->blocked_carve = carve;
       GPR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_bsm, k, 1024 / g->blocked_ctas, smem));
       if (per_bsm >= g->blocked_ctas || g->blocked_ctas == 1) break;
       g->blocked_ctas = 1;
@@ -1259,6 +1262,10 @@ int solve_phase(gpr_multigraph *g, float *d_scores, const gpr_pr_opts &o, bool b
     }
   } else if (max_cap > 0 && blocked) {
     void *args[] = {&a};
+    // a preference of the function, not of the launch: this batch's
+    GPR_CUDA(cudaFuncSetAttribute(multi_blocked_kernel(g->blocked_ctas),
+                                  cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  g->blocked_carve));
     cudaError_t e = cudaLaunchCooperativeKernel(
         multi_blocked_kernel(g->blocked_ctas), dim3(g->grid_blocked),
         dim3(1024 / g->blocked_ctas), args, 8 * (size_t)g->B.R, st);

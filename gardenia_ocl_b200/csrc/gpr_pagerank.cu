@@ -815,8 +815,11 @@ int create_impl(int m, long long nnz, const int *any_rowptr, const int *any_col,
   for (int v = 0; v < kNumKernels; ++v) {
     int per_sm = 0;
     const size_t smem = (size_t)hot_entries(g, v) * kKernels[v].elem;
+    // the attribute belongs to the function: the same for every graph, or a small
+    // graph's would refuse a larger one's launches
     GPR_CUDA(cudaFuncSetAttribute(kKernels[v].persistent,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kKernels[v].hot_bytes));
     GPR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kKernels[v].persistent,
                                                            kHotBlock, smem));
     if (per_sm < kKernels[v].ctas_per_sm) g->hot_ok = false;
@@ -849,8 +852,10 @@ int create_impl(int m, long long nnz, const int *any_rowptr, const int *any_col,
       GPR_CUDA(cudaFuncGetAttributes(&fa, k));
       const long long need = (long long)g->blocked_ctas * (smem + (long long)fa.sharedSizeBytes + 1024);
       const int carve = (int)std::min<long long>(100, gpr::ceil_div(100 * need, smem_sm));
-      GPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      GPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    8 * gpr::kBlockedMaxRows));
       GPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
+      g->blocked_carve = carve;
       GPR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
           &per_sm, k, 1024 / g->blocked_ctas, smem));
       if (per_sm >= g->blocked_ctas || g->blocked_ctas == 1) break;
@@ -1012,6 +1017,10 @@ int solve_impl(gpr_graph *g, float *d_scores, const gpr_pr_opts &o, int ki, gpr_
   GPR_CUDA(cudaEventRecord(g->e2, st));
   if (o.max_iter > 0 && blocked) {
     void *args[] = {&a};
+    // a preference of the function, not of the launch: this graph's
+    GPR_CUDA(cudaFuncSetAttribute(blocked_kernel(g->blocked_ctas),
+                                  cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  g->blocked_carve));
     cudaError_t e = cudaLaunchCooperativeKernel(blocked_kernel(g->blocked_ctas),
                                                 dim3(g->grid_blocked),
                                                 dim3(1024 / g->blocked_ctas), args,

@@ -224,7 +224,8 @@ int push_impl(gpr_graph *g, float *any_scores, const gpr_pr_opts &o, gpr_pr_stat
   const int hot = std::min(gpr::kHotDefault, m);
   const size_t smem = sizeof(float) * (size_t)hot;
   GPR_CUDA(cudaFuncSetAttribute((const void *)k_pr_push,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(float) * gpr::kHotDefault));
   GPR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k_pr_push,
                                                          kPushBlock, smem));
   if (!coop || per_sm < 1) {

@@ -280,3 +280,18 @@ def test_units_dealt_to_ctas(G, O, m):
     assert st.iterations == 5
     assert np.array_equal(s, ref)
     np.testing.assert_allclose(hist, ref_hist, rtol=1e-12)
+
+
+@pytest.mark.parametrize("blocked", [False, True])
+def test_large_graph_solved_after_a_small_one_was_made(G, O, blocked):
+    # Shared-memory limits belong to a kernel, not to a graph: a graph with a
+    # smaller staged prefix or smaller blocks does not take them from another.
+    big, small = O.rmat_graph(16, 8, seed=3), O.rmat_graph(9, 8, seed=4)
+    form = G.FORM_BLOCKED if blocked else G.FORM_EXACT
+    rows = 4096 if blocked else 0
+    with G.Graph(*big, blocked=blocked, block_rows=rows) as g:
+        ref, _ = g.pagerank(tol=0.0, max_iter=3, form=form)
+        with G.Graph(*small, blocked=blocked) as g2:
+            g2.pagerank(tol=0.0, max_iter=3, form=form)
+            s, _ = g.pagerank(tol=0.0, max_iter=3, form=form)
+    assert np.array_equal(s, ref)
