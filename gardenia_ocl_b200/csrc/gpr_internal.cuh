@@ -283,8 +283,8 @@ struct gpr_graph {
   int *b_pkr[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   int b_npkr[6] = {-1, -1, -1, -1, -1, -1};
   long long b_pkwr[6] = {0, 0, 0, 0, 0, 0};
-  // Push solver: edges sorted by source and the per-vertex accumulators,
-  // built on first use.
+  // Push solver without blocks: edges sorted by source and the per-vertex
+  // accumulators, built on first use.
   int *push_src = nullptr, *push_dst = nullptr;
   float *push_sum = nullptr;
   // Graph mode: the instantiated sweep-loop graph and the kernel and
@@ -296,6 +296,8 @@ struct gpr_graph {
   // grid and co-residency, the tile-queue heads and the largest |score|.
   gpr::BlockedLayout B;
   bool has_blocked = false, blocked_ok = false;
+  bool has_push = false;       // B was built by the push solver (pull solves do not use it)
+  bool push_plain = false;     // B could not be built for the push solver
   int grid_blocked = 0, blocked_ctas = 1;  // blocked-form CTAs: total, per SM
   int blocked_carve = 0;       // shared-memory share of the SM for them, percent
   int *tq = nullptr;
@@ -304,6 +306,11 @@ struct gpr_graph {
 };
 
 namespace gpr {
+// The push solver's solve in the blocked form (gpr_pagerank.cu).  kPushFallback: the
+// form does not apply (a non-finite score, no co-resident grid); nothing was done.
+constexpr int kPushFallback = 101;
+int push_blocked(gpr_graph *g, float *any_scores, const gpr_pr_opts &opts, gpr_pr_stats *stats);
+
 constexpr int kZeroRowsPerUnit = 128;  // rows per zero-in-degree work unit
 constexpr int kSellMaxDefault = 64;    // SpMV: row length bound of the SELL bin;
                                        // PR: max edges per lane in a SELL slice

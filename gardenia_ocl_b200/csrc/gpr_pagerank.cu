@@ -697,6 +697,51 @@ void destroy(gpr_graph *g) {
   delete g;
 }
 
+// Grid and shared-memory carveout of the blocked kernel for g->B, and the buffers it
+// needs beside the exact-order form's.
+int setup_blocked(gpr_graph *g, int sms) {
+  int smem_sm = 0;
+  GPR_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor,
+                                  g->device));
+  // Two 512-thread CTAs per SM (one gathers while the other closes a tile)
+  // when both fit beside an L1 of about half the SM's 256 KB, else one
+  // 1024-thread CTA: the gathers' L1 line hits are worth more than the
+  // overlap (RMAT scale 24 with 12288-row blocks: 2x slower sweeps with
+  // two CTAs and a 28 KB L1).
+  g->blocked_ctas = gpr::blocked_ctas_per_sm(g->B.R);
+  int per_sm = 0;
+  for (;;) {
+    // the smallest shared-memory carveout that holds the CTAs: the rest of
+    // the SM's 256 KB stays L1
+    const void *k = blocked_kernel(g->blocked_ctas);
+    const int smem = 8 * g->B.R;
+    cudaFuncAttributes fa;
+    GPR_CUDA(cudaFuncGetAttributes(&fa, k));
+    const long long need = (long long)g->blocked_ctas * (smem + (long long)fa.sharedSizeBytes + 1024);
+    const int carve = (int)std::min<long long>(100, gpr::ceil_div(100 * need, smem_sm));
+    GPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  8 * gpr::kBlockedMaxRows));
+    GPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
+    g->blocked_carve = carve;
+    GPR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &per_sm, k, 1024 / g->blocked_ctas, smem));
+    if (per_sm >= g->blocked_ctas || g->blocked_ctas == 1) break;
+    g->blocked_ctas = 1;
+  }
+  g->blocked_ok = g->coop && per_sm >= g->blocked_ctas;
+  g->grid_blocked = sms * g->blocked_ctas;
+  g->max_grid = std::max(g->max_grid, g->grid_blocked);
+  GPR_TRY(gpr::dalloc(&g->tq, 2, "tile queue"));
+  GPR_TRY(gpr::dalloc(&g->fx_max, 1, "largest score"));
+  return GPR_OK;
+}
+
+// Rows per block when the caller gave none: about two blocks per SM.
+int default_block_rows(int n_nz, int sms) {
+  return (int)std::min<long long>(
+      gpr::kBlockedRows, std::max<long long>(256, gpr::ceil_div((long long)n_nz, 2LL * sms)));
+}
+
 int create_impl(int m, long long nnz, const int *any_rowptr, const int *any_col,
                 const int *any_outdeg, int lane_max, int chunk_min, int chunk, int hot_max,
                 bool keep_csr, bool blocked, int block_rows, int tile_words, int blocked_long,
@@ -760,16 +805,12 @@ int create_impl(int m, long long nnz, const int *any_rowptr, const int *any_col,
     if (ev_col) cudaEventDestroy(ev_col);
   }
   if (rc == GPR_OK && blocked) {
-    // Default rows per block: about two blocks per SM.  Default tile size:
-    // whole blocks up to 1M words (a multi-tile block adds one 8-byte atomic
+    // Default tile size: whole blocks up to 1M words (a multi-tile block adds one 8-byte atomic
     // per row and tile); the builder halves the tiles that would end the
     // sweep late.
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, g->device);
-    if (block_rows == 0)
-      block_rows = (int)std::min<long long>(
-          gpr::kBlockedRows,
-          std::max<long long>(256, gpr::ceil_div((long long)g->L.n_nz, 2LL * nsm)));
+    if (block_rows == 0) block_rows = default_block_rows(g->L.n_nz, nsm);
     int row0 = 0, n_chunks = 0;
     rc = gpr::blocked_split(g->L, (const int *)rp,
                             blocked_long > 0 ? std::max(blocked_long, chunk_min) : 0, block_rows,
@@ -832,41 +873,7 @@ int create_impl(int m, long long nnz, const int *any_rowptr, const int *any_col,
   g->grid_step = (int)step;
   g->max_grid = g->grid_step;
   for (int v = 0; v < kNumKernels; ++v) g->max_grid = std::max(g->max_grid, g->grid_hot[v]);
-  if (g->has_blocked) {
-    int smem_sm = 0;
-    GPR_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor,
-                                    g->device));
-    // Two 512-thread CTAs per SM (one gathers while the other closes a tile)
-    // when both fit beside an L1 of about half the SM's 256 KB, else one
-    // 1024-thread CTA: the gathers' L1 line hits are worth more than the
-    // overlap (RMAT scale 24 with 12288-row blocks: 2x slower sweeps with
-    // two CTAs and a 28 KB L1).
-    g->blocked_ctas = gpr::blocked_ctas_per_sm(g->B.R);
-    int per_sm = 0;
-    for (;;) {
-      // the smallest shared-memory carveout that holds the CTAs: the rest of
-      // the SM's 256 KB stays L1
-      const void *k = blocked_kernel(g->blocked_ctas);
-      const int smem = 8 * g->B.R;
-      cudaFuncAttributes fa;
-      GPR_CUDA(cudaFuncGetAttributes(&fa, k));
-      const long long need = (long long)g->blocked_ctas * (smem + (long long)fa.sharedSizeBytes + 1024);
-      const int carve = (int)std::min<long long>(100, gpr::ceil_div(100 * need, smem_sm));
-      GPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    8 * gpr::kBlockedMaxRows));
-      GPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-      g->blocked_carve = carve;
-      GPR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &per_sm, k, 1024 / g->blocked_ctas, smem));
-      if (per_sm >= g->blocked_ctas || g->blocked_ctas == 1) break;
-      g->blocked_ctas = 1;
-    }
-    g->blocked_ok = g->coop && per_sm >= g->blocked_ctas;
-    g->grid_blocked = sms * g->blocked_ctas;
-    g->max_grid = std::max(g->max_grid, g->grid_blocked);
-    GPR_TRY(gpr::dalloc(&g->tq, 2, "tile queue"));
-    GPR_TRY(gpr::dalloc(&g->fx_max, 1, "largest score"));
-  }
+  if (g->has_blocked) GPR_TRY(setup_blocked(g, sms));
   GPR_TRY(gpr::dalloc(&g->cta_err, 2 * (size_t)g->max_grid, "cta residuals"));
   g->err_cap = 128;
   GPR_TRY(gpr::dalloc(&g->err_hist, (size_t)g->err_cap, "residual history"));
@@ -1082,8 +1089,10 @@ int solve_impl(gpr_graph *g, float *d_scores, const gpr_pr_opts &o, int ki, gpr_
   return GPR_OK;
 }
 
+// `push`: the push solver's solve in the blocked form (kBlockedFallback: not
+// possible, nothing changed).
 int pagerank_impl(gpr_graph *g, float *any_scores, const gpr_pr_opts *opts_in,
-                  gpr_pr_stats *stats) {
+                  gpr_pr_stats *stats, bool push = false) {
   gpr_pr_opts o;
   if (opts_in) o = *opts_in;
   else gpr_pr_opts_default(&o);
@@ -1143,12 +1152,12 @@ int pagerank_impl(gpr_graph *g, float *any_scores, const gpr_pr_opts *opts_in,
   }
   int rc = GPR_OK;
   const bool use_blocked =
-      o.precision == GPR_PREC_FP32 && g->has_blocked && g->blocked_ok &&
-      o.loop != GPR_LOOP_GRAPH && o.form != GPR_FORM_EXACT &&
-      (o.form == GPR_FORM_BLOCKED || g->L.nnz >= gpr::kBlockedAutoMinEdges);
+      push || (o.precision == GPR_PREC_FP32 && g->has_blocked && g->blocked_ok &&
+               o.loop != GPR_LOOP_GRAPH && o.form != GPR_FORM_EXACT &&
+               (o.form == GPR_FORM_BLOCKED || g->L.nnz >= gpr::kBlockedAutoMinEdges));
   if (use_blocked) {
     rc = solve_impl(g, d_scores, o, 0, &st_local, true);
-    if (rc == kBlockedFallback) {
+    if (rc == kBlockedFallback && !push) {
       if (o.form == GPR_FORM_BLOCKED) {
         gpr::set_error("gpr_pagerank: GPR_FORM_BLOCKED needs finite scores and a "
                        "co-resident grid");
@@ -1186,7 +1195,66 @@ int pagerank_impl(gpr_graph *g, float *any_scores, const gpr_pr_opts *opts_in,
   return rc;
 }
 
+__global__ void k_identity(int m, int *perm) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < m) perm[i] = i;
+}
+
+// The blocked layout of a graph created without it, from its relabelled CSR.
+int build_push_layout(gpr_graph *g) {
+  int sms = 148;
+  GPR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
+  PrLayout L = g->L;  // rows are in the relabelled order already
+  int *perm = nullptr;
+  GPR_TRY(gpr::dalloc(&perm, (size_t)L.m, "identity"));
+  k_identity<<<grid_for(L.m), 256, 0, g->st>>>(L.m, perm);
+  L.perm = perm;
+  const int R = default_block_rows(L.n_nz, sms);
+  int row0 = 0, n_chunks = 0;
+  int rc = GPR_CUDA_RC(cudaGetLastError());
+  if (rc == GPR_OK) rc = gpr::blocked_split(L, L.csr_ptr, 0, R, &row0, &n_chunks, g->st);
+  if (rc == GPR_OK)
+    rc = gpr::build_blocked_layout(L.m, L.nnz, L.csr_ptr, L.csr_col, L, row0, n_chunks, R,
+                                   gpr::kTileWordsDefault, gpr::kRunWords,
+                                   sms * gpr::blocked_ctas_per_sm(R), &g->B, g->st);
+  gpr::dfree(perm);
+  GPR_TRY(rc);
+  const int grid = g->max_grid;
+  double *part = nullptr;
+  rc = setup_blocked(g, sms);
+  if (rc == GPR_OK && g->max_grid > grid) {  // more CTAs than there are residual partials
+    rc = gpr::dalloc(&part, 2 * (size_t)g->max_grid, "cta residuals");
+    if (rc == GPR_OK) {
+      gpr::dfree(g->cta_err);
+      g->cta_err = part;
+    }
+  }
+  if (rc != GPR_OK) {
+    g->max_grid = grid;
+    g->blocked_ok = false;
+  }
+  g->has_push = rc == GPR_OK;
+  return rc;
+}
+
 }  // namespace
+
+int gpr::push_blocked(gpr_graph *g, float *any_scores, const gpr_pr_opts &opts,
+                      gpr_pr_stats *stats) {
+  if (!g->has_blocked && !g->has_push && !g->push_plain) {
+    // The build needs more scratch than the plain push's edge list (24 bytes an
+    // edge beside the sort against 12) and has a limit of its own on words.
+    const int rc = build_push_layout(g);
+    if (rc == GPR_ENOMEM || rc == GPR_EINVAL) g->push_plain = true;
+    else GPR_TRY(rc);
+  }
+  if (g->push_plain || !g->blocked_ok) return kPushFallback;
+  gpr_pr_opts o = opts;
+  o.variant = 0;
+  o.form = GPR_FORM_AUTO;
+  const int rc = pagerank_impl(g, any_scores, &o, stats, true);
+  return rc == kBlockedFallback ? kPushFallback : rc;
+}
 
 extern "C" {
 

@@ -214,9 +214,12 @@ int gpr_ppr(gpr_graph *g, int k, const int *h_seeds, float *any_x,
  * The reference's push variants (src/pr/scatter.cu:16-41, lb.cu:20-82)
  * scatter each source's contribution to its out-neighbours with atomic adds.
  * Same recurrence and stop rule as gpr_pagerank (so the two directions solve
- * the same problem); edges sorted by source, hot destinations accumulated in
- * shared memory, one persistent launch.  Atomic adds make the last bits of
- * the result vary from run to run.  The graph must be created with
+ * the same problem).  The first call builds the blocked layout (edges in source
+ * order, cut by destination block; see gpr_form) and every solve adds the
+ * contributions to their destinations' accumulators in shared memory, in 64-bit
+ * fixed point: deterministic.  With a non-finite initial score, or without the
+ * scratch for that layout, edges sorted by source add one by one in FP32, and the
+ * last bits of the result vary from run to run.  The graph must be created with
  * GPR_LAYOUT_PUSH (or GPR_LAYOUT_BATCHED); FP32 only. */
 int gpr_pagerank_push(gpr_graph *g, float *any_scores, const gpr_pr_opts *opts,
                       gpr_pr_stats *stats);

@@ -1,7 +1,8 @@
-"""Push-style PageRank (atomic scatter over a source-sorted edge list) on the
+"""Push-style PageRank (a scatter in source order into destination blocks, or edge by
+edge with atomic float adds where a score is not finite) on the
 GPU, held to the plain path's bar against the reference's pull recurrence
 (1e-6 per vertex plus the reference's own float error on hub rows, sweeps
-within one).  Atomic adds make the last bits vary between runs."""
+within one)."""
 import numpy as np
 import pytest
 
@@ -64,3 +65,42 @@ def test_push_barrier_timeout(G, O):
         assert e.value.status == G.GPR_ETIMEOUT
         s, st = g.pagerank_push(tol=1e-6, max_iter=10)
         assert st.iterations > 0
+
+
+@pytest.mark.parametrize("maker", ["rmat", "star", "no_edges", "one_edge"])
+def test_push_in_blocks(G, O, maker):
+    """The push solver's blocked solve gives the bits of the blocked pull solve on a
+    layout built at creation, the same twice, and leaves the graph's own pull
+    solves as they were."""
+    rp, col, od = {"rmat": lambda: O.rmat_graph(13, 16, seed=5), "star": lambda: star(5000),
+                   "no_edges": lambda: (np.zeros(301, np.int32), np.zeros(0, np.int32),
+                                        np.zeros(300, np.int32)),
+                   "one_edge": lambda: (np.array([0, 0, 1], np.int32), np.zeros(1, np.int32),
+                                        np.array([1, 0], np.int32))}[maker]()
+    kw = dict(tol=0.0, max_iter=6)
+    with G.Graph(rp, col, od, blocked=True) as g:
+        ref, _ = g.pagerank(form=G.FORM_BLOCKED, **kw)
+    with G.Graph(rp, col, od, push=True) as g:
+        before, _ = g.pagerank(**kw)
+        a, st = g.pagerank_push(**kw)
+        b, _ = g.pagerank_push(**kw)
+        after, _ = g.pagerank(**kw)
+    assert st.iterations == 6
+    assert np.array_equal(a, ref) and np.array_equal(a, b)
+    assert np.array_equal(before, after)
+
+
+def test_push_non_finite_scores(G, O):
+    """An infinite score cannot be held in fixed point: those edges add one by one, and
+    the infinities reach the vertices that the reference's reach."""
+    rp, col, od = erdos_renyi(3000, 6, seed=9)
+    s0 = np.full(3000, np.float32(1 / 3000))
+    s0[int(np.argmax(od))] = np.inf
+    ref, _, _ = O.pr_plain_f32(rp, col, od, scores=s0, tol=0.0, max_iter=2)
+    with G.Graph(rp, col, od, push=True) as g:
+        g.pagerank_push(tol=0.0, max_iter=2)
+        s, st = g.pagerank_push(s0.copy(), tol=0.0, max_iter=2)
+    fin = np.isfinite(ref)
+    assert st.iterations == 2 and not fin.all()
+    assert np.array_equal(fin, np.isfinite(s))
+    assert np.abs(s[fin] - ref[fin]).max() <= 1e-6
