@@ -198,8 +198,8 @@ void free_blocked_layout(BlockedLayout *B) {
   *B = BlockedLayout();
 }
 
-int blocked_split(const PrLayout &L, const int *d_rowptr, int long_min, int R, int *row0,
-                  int *n_chunks, cudaStream_t st) {
+int blocked_split(const PrLayout &L, const int *d_rowptr, int long_min, int least, int R,
+                  int *row0, int *n_chunks, cudaStream_t st) {
   *row0 = 0;
   *n_chunks = 0;
   if (L.n_long == 0) return GPR_OK;
@@ -228,7 +228,7 @@ int blocked_split(const PrLayout &L, const int *d_rowptr, int long_min, int R, i
   } else {
     long long win = 0;  // in-edges of rows [cnt, cnt + R)
     for (int j = 0; j < std::min(n, R); ++j) win += deg[j];
-    while (cnt < L.n_long && 8LL * deg[cnt] > win) {
+    while (cnt < L.n_long && deg[cnt] > least && 8LL * deg[cnt] > win) {
       win -= deg[cnt];
       if (cnt + R < n) win += deg[cnt + R];
       ++cnt;

@@ -90,6 +90,8 @@ struct PrLayout {
   int *long_col = nullptr;        // relabelled sources of the long rows
   int *row_cbeg = nullptr;        // [n_long+1] first chunk of each long row
   int *chunk_row = nullptr;       // [n_chunks] row of each chunk
+  int4 *chunk_desc = nullptr;     // [n_chunks] {row, first edge / 4, edges, first chunk of the
+                                  // row or -1 when it has one}: one load per chunk
   long long *slice_ptr = nullptr; // [n_slices+1] offsets into sell_col
   int *sell_col = nullptr;        // relabelled sources, SELL-32 column-major
   int *csr_ptr = nullptr;         // [m+1] relabelled CSR (batched solvers only)
@@ -152,11 +154,12 @@ struct BlockedLayout {
 
 // Rows of the blocked form that stay chunked: the first *row0 rows of the
 // exact-order layout's chunked rows [0, L.n_long), either those with more than
-// long_min in-edges or, when long_min is 0, those holding more than 1/8 of the
-// in-edges of the R rows that start at them; and their *n_chunks chunks.
+// long_min in-edges or, when long_min is 0, those with more than `least` that hold
+// more than 1/8 of the in-edges of the R rows that start at them; and their
+// *n_chunks chunks.
 // Synchronizes st.
-int blocked_split(const PrLayout &L, const int *d_rowptr, int long_min, int R, int *row0,
-                  int *n_chunks, cudaStream_t st);
+int blocked_split(const PrLayout &L, const int *d_rowptr, int long_min, int least, int R,
+                  int *row0, int *n_chunks, cudaStream_t st);
 int build_blocked_layout(int m, long long nnz, const int *d_rowptr, const int *d_col,
                          const PrLayout &L, int row0, int n_chunks, int R, int tile_slots,
                          int run_words, int workers, BlockedLayout *B, cudaStream_t st);
@@ -318,7 +321,31 @@ constexpr int kChunkMinDefault = 4096; // PR: rows with more in-edges are chunke
 constexpr int kChunkDefault = 4096;    // edges per long-row chunk (multiple of 128)
 constexpr int kBlock = 256;            // threads per CTA of the per-sweep kernels
 constexpr int kHotDefault = 32768;     // contributions staged in shared memory (128 KB)
+constexpr int kHotMin = 4096;
 constexpr int kHotMax = 56832;         // 222 KB: the most one CTA may take
+
+// Defaults of the chunk size (and of the in-degree above which rows are chunked)
+// and of the staged prefix for a graph of nnz edges.  A chunk is about one warp's
+// share of the edges (148 SMs x 32 warps), so that no warp works on its chunk while
+// the others are done; below 2^19 edges a sweep is a few dependent loads, and the
+// chunks' combination costs more than it saves.  Sweep loop, RMAT, chunks of 512 /
+// 1024 / 2048 / 4096 edges: 10,007 vertices (0.15M edges) 101 / - / - / 91 us, 65,536
+// (0.95M) 236 / 238 / - / 293, 250,007 (3.6M) 678 / 658 / - / 777, 1,000,003 (15M)
+// 2078 / 1751 / 1743 / 1806, 3,000,017 (34M) 4293 / 3821 / 3781 / 3771.  Staging costs
+// every SM the prefix once a sweep: 65,536 vertices with 4096 / 16384 / 32768 staged
+// 208 / 212 / 238 us, 250,007 770 / 729 / 764; 10,007 with 4096 / all staged 168 / 160 us
+// per call.
+inline int default_chunk(long long nnz) {
+  if (nnz < (1 << 19)) return kChunkDefault;
+  int c = 512;
+  while (c < kChunkDefault && 2LL * c * 4736 <= nnz) c *= 2;
+  return c;
+}
+inline int default_hot(long long nnz) {
+  if (nnz < (1 << 19)) return kHotDefault;
+  const long long h = nnz / 200 / 4 * 4;
+  return (int)(h < kHotMin ? kHotMin : h > kHotDefault ? kHotDefault : h);
+}
 
 __host__ __device__ inline long long ceil_div(long long a, long long b) {
   return (a + b - 1) / b;

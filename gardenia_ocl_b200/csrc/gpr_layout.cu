@@ -83,20 +83,24 @@ __global__ void k_fill_chunk_row(int n_long, const int *__restrict__ cbeg, int *
     for (int c = cbeg[r] + lane; c < cbeg[r + 1]; c += 32) chunk_row[c] = (int)r;
 }
 
-// One warp per long row: relabelled sources, padded with the sentinel m.
-__global__ void k_fill_long(int n_long, int m, const int *__restrict__ perm,
+// One warp per chunk of a long row: its descriptor and its relabelled sources,
+// padded with the sentinel m.
+__global__ void k_fill_long(int n_chunks, int chunk, int m, const int *__restrict__ chunk_row,
+                            const int *__restrict__ cbeg, const int *__restrict__ perm,
                             const int *__restrict__ inv, const int *__restrict__ rowptr,
                             const int *__restrict__ col, const long long *__restrict__ lptr,
-                            int *long_col) {
+                            int4 *desc, int *long_col) {
   int lane = threadIdx.x & 31;
   long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long r = w; r < n_long; r += nw) {
-    int o = perm[r];
-    long long sb = rowptr[o];
-    long long deg = rowptr[o + 1] - sb;
-    long long db = lptr[r], plen = lptr[r + 1] - db;
-    for (long long k = lane; k < plen; k += 32)
+  for (long long c = w; c < n_chunks; c += nw) {
+    const int r = chunk_row[c], o = perm[r], cb = cbeg[r];
+    const long long sb = rowptr[o], deg = rowptr[o + 1] - sb;
+    const long long db = lptr[r], plen = lptr[r + 1] - db;
+    const long long k0 = (c - cb) * chunk, k1 = min(plen, k0 + chunk);
+    if (lane == 0)
+      desc[c] = make_int4(r, (int)((db + k0) >> 2), (int)(k1 - k0), cbeg[r + 1] - cb == 1 ? -1 : cb);
+    for (long long k = k0 + lane; k < k1; k += 32)
       long_col[db + k] = (k < deg) ? inv[col[sb + k]] : m;
   }
 }
@@ -351,6 +355,7 @@ int build_pr_layout(int m, long long nnz, const int *d_rowptr, const int *d_col,
   }
   GPR_TRY(dalloc(&L->long_col, (size_t)L->long_elems, "long rows"));
   GPR_TRY(dalloc(&L->chunk_row, (size_t)L->n_chunks, "chunk rows"));
+  GPR_TRY(dalloc(&L->chunk_desc, (size_t)L->n_chunks, "chunk descriptors"));
   const unsigned g_long = std::min(grid_for(32LL * L->n_long), 148u * 32u);
   if (L->n_long > 0) k_fill_chunk_row<<<g_long, 256, 0, st>>>(L->n_long, L->row_cbeg, L->chunk_row);
 
@@ -372,8 +377,9 @@ int build_pr_layout(int m, long long nnz, const int *d_rowptr, const int *d_col,
     GPR_TRY(validate_cols(nnz, m, d_col, st));
   }
   if (L->n_long > 0)
-    k_fill_long<<<g_long, 256, 0, st>>>(L->n_long, m, L->perm, inv, d_rowptr, d_col, L->long_ptr,
-                                        L->long_col);
+    k_fill_long<<<std::min(grid_for(32LL * L->n_chunks), 148u * 32u), 256, 0, st>>>(
+        L->n_chunks, chunk, m, L->chunk_row, L->row_cbeg, L->perm, inv, d_rowptr, d_col,
+        L->long_ptr, L->chunk_desc, L->long_col);
   if (L->n_slices > 0)
     k_fill_sell<<<grid_for(32LL * L->n_slices), 256, 0, st>>>(
         L->n_slices, m, C, L->perm, inv, d_rowptr, d_col, sdeg, L->slice_ptr, L->sell_col);
@@ -390,7 +396,7 @@ int build_pr_layout(int m, long long nnz, const int *d_rowptr, const int *d_col,
   GPR_CUDA(cudaGetLastError());
   GPR_CUDA(cudaStreamSynchronize(st));
   L->device_bytes = 4LL * (2LL * m) + 8LL * (L->n_long + 1) + 4LL * L->long_elems +
-                    4LL * (L->n_long + 1) + 4LL * L->n_chunks + 8LL * (L->n_slices + 1) +
+                    4LL * (L->n_long + 1) + 20LL * L->n_chunks + 8LL * (L->n_slices + 1) +
                     4LL * L->sell_elems + (keep_csr ? 4LL * (m + 1) + 4LL * nnz : 0);
   return GPR_OK;
 }
@@ -402,6 +408,7 @@ void free_pr_layout(PrLayout *L) {
   dfree(L->long_col);
   dfree(L->row_cbeg);
   dfree(L->chunk_row);
+  dfree(L->chunk_desc);
   dfree(L->slice_ptr);
   dfree(L->sell_col);
   dfree(L->csr_ptr);

@@ -866,6 +866,8 @@ int build_multi(gpr_multigraph *g, const int *h_voff, const int *d_rowptr, const
     lane_max[r] = lo && lo->sell_max ? lo->sell_max : gpr::kSellMaxDefault;
     chunk_min[r] = lo && lo->chunk_min ? lo->chunk_min : gpr::kChunkMinDefault;
     chunk[r] = lo && lo->chunk ? lo->chunk : gpr::kChunkDefault;
+    if (!lo || (!lo->chunk && !lo->chunk_min))  // as the single-graph layout's
+      chunk[r] = chunk_min[r] = gpr::default_chunk(eoff[ug + 1] - eoff[ug]);
     int *t = th.data() + 8 * (size_t)r;
     t[0] = chunk_min[r];
     for (int lw = 4; lw >= 0; --lw) t[5 - lw] = (int)std::min<long long>((long long)lane_max[r] << lw, chunk_min[r]);

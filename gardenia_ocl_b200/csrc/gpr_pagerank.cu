@@ -47,6 +47,7 @@ struct PrArgs {
   const int *long_col;
   const int *row_cbeg;
   const int *chunk_row;
+  const int4 *chunk_desc;
   const long long *slice_ptr;
   const int *sell_col;
   const int *outdeg;
@@ -98,17 +99,15 @@ __device__ __forceinline__ double row_update(const PrArgs &a, int r, float sum, 
 template <int U4, typename Gather, typename T>
 __device__ __forceinline__ double do_chunk(const PrArgs &a, const Gather &gat, T *cout, int c,
                                            int lane, const Policies &pol) {
-  const int r = a.chunk_row[c];
-  const int cb = a.row_cbeg[r];
-  const int nc = a.row_cbeg[r + 1] - cb;
+  const int4 d = __ldg(a.chunk_desc + c);
+  const int r = d.x, cb = d.w;
   float so = 0.f;
   int od = 1;
   if (lane == 0) {
     so = ld_f32_stream(a.s + r, pol.stream);
     od = ld_s32_stream(a.outdeg + r, pol.stream);
   }
-  const long long b = a.long_ptr[r] + (long long)(c - cb) * a.chunk;
-  const long long e = min(b + (long long)a.chunk, a.long_ptr[r + 1]);
+  const long long b = 4LL * d.y, e = b + d.z;
   float acc = 0.f;
   for (long long k0 = b + 4 * lane; k0 < e; k0 += 128 * U4) {
     int4 q[U4];
@@ -128,7 +127,8 @@ __device__ __forceinline__ double do_chunk(const PrArgs &a, const Gather &gat, T
     for (int i = 0; i < 4 * U4; ++i) acc += v[i];
   }
   acc = warp_sum(acc);
-  if (nc == 1) return lane == 0 ? row_update(a, r, acc, so, od, cout, pol) : 0.0;
+  if (cb < 0) return lane == 0 ? row_update(a, r, acc, so, od, cout, pol) : 0.0;
+  const int nc = __ldg(a.row_cbeg + r + 1) - cb;
   int last = 0;
   if (lane == 0) {
     a.partial[c] = acc;
@@ -635,6 +635,7 @@ PrArgs make_args(gpr_graph *g, const gpr_pr_opts &o, int ki) {
   a.long_col = L.long_col;
   a.row_cbeg = L.row_cbeg;
   a.chunk_row = L.chunk_row;
+  a.chunk_desc = L.chunk_desc;
   a.slice_ptr = L.slice_ptr;
   a.sell_col = L.sell_col;
   a.outdeg = L.outdeg;
@@ -745,7 +746,7 @@ int default_block_rows(int n_nz, int sms) {
 int create_impl(int m, long long nnz, const int *any_rowptr, const int *any_col,
                 const int *any_outdeg, int lane_max, int chunk_min, int chunk, int hot_max,
                 bool keep_csr, bool blocked, int block_rows, int tile_words, int blocked_long,
-                gpr_graph *g) {
+                int split_min, gpr_graph *g) {
   GPR_CUDA(cudaGetDevice(&g->device));
   GPR_CUDA(cudaStreamCreateWithFlags(&g->st, cudaStreamNonBlocking));
   g->own_stream = true;
@@ -813,8 +814,8 @@ int create_impl(int m, long long nnz, const int *any_rowptr, const int *any_col,
     if (block_rows == 0) block_rows = default_block_rows(g->L.n_nz, nsm);
     int row0 = 0, n_chunks = 0;
     rc = gpr::blocked_split(g->L, (const int *)rp,
-                            blocked_long > 0 ? std::max(blocked_long, chunk_min) : 0, block_rows,
-                            &row0, &n_chunks, st);
+                            blocked_long > 0 ? std::max(blocked_long, split_min) : 0, split_min,
+                            block_rows, &row0, &n_chunks, st);
     if (tile_words == 0) tile_words = gpr::kTileWordsDefault;
     if (rc == GPR_OK)
       rc = gpr::build_blocked_layout(m, nnz, (const int *)rp, (const int *)cp, g->L, row0,
@@ -1212,7 +1213,8 @@ int build_push_layout(gpr_graph *g) {
   const int R = default_block_rows(L.n_nz, sms);
   int row0 = 0, n_chunks = 0;
   int rc = GPR_CUDA_RC(cudaGetLastError());
-  if (rc == GPR_OK) rc = gpr::blocked_split(L, L.csr_ptr, 0, R, &row0, &n_chunks, g->st);
+  if (rc == GPR_OK) rc = gpr::blocked_split(L, L.csr_ptr, 0, gpr::kChunkMinDefault, R, &row0, &n_chunks,
+                                               g->st);
   if (rc == GPR_OK)
     rc = gpr::build_blocked_layout(L.m, L.nnz, L.csr_ptr, L.csr_col, L, row0, n_chunks, R,
                                    gpr::kTileWordsDefault, gpr::kRunWords,
@@ -1268,6 +1270,10 @@ int gpr_graph_create_ex(int m, long long nnz, const int *any_rowptr, const int *
   GPR_ENTRY_BEGIN
   int lane_max = gpr::kSellMaxDefault, chunk = gpr::kChunkDefault,
       chunk_min = gpr::kChunkMinDefault, hot_max = gpr::kHotDefault;
+  if (!lopts || (!lopts->chunk && !lopts->chunk_min)) chunk = chunk_min = gpr::default_chunk(nnz);
+  hot_max = gpr::default_hot(nnz);
+  // rows the blocked form may leave in chunks: above the caller's chunk_min
+  const int split_min = lopts && lopts->chunk_min ? lopts->chunk_min : gpr::kChunkMinDefault;
   if (lopts && lopts->sell_max) lane_max = lopts->sell_max;
   if (lopts && lopts->chunk) chunk = lopts->chunk;
   if (lopts && lopts->chunk_min) chunk_min = lopts->chunk_min;
@@ -1306,7 +1312,8 @@ int gpr_graph_create_ex(int m, long long nnz, const int *any_rowptr, const int *
   const bool keep_csr = lopts && (lopts->flags & (GPR_LAYOUT_BATCHED | GPR_LAYOUT_PUSH));
   const bool blocked = lopts && (lopts->flags & GPR_LAYOUT_BLOCKED);
   int rc = create_impl(m, nnz, any_rowptr, any_col, any_outdeg, lane_max, chunk_min, chunk,
-                       hot_max, keep_csr, blocked, block_rows, tile_words, blocked_long, g);
+                       hot_max, keep_csr, blocked, block_rows, tile_words, blocked_long,
+                       split_min, g);
   if (rc != GPR_OK) {
     destroy(g);
     return rc;

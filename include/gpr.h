@@ -136,10 +136,14 @@ enum {
 typedef struct {
   int sell_max;   /* max edges per lane in a SELL slice: rows of in-degree <= sell_max get
                      one lane, wider rows 2..32 lanes (default 64) */
-  int chunk;      /* edges per long-row chunk, multiple of 128 (default 4096) */
-  int chunk_min;  /* rows with more in-edges than this are cut into chunks (default 4096) */
+  int chunk;      /* edges per long-row chunk, multiple of 128 (default 4096; when chunk_min
+                     is 0 too and the graph has 2^19 edges or more, about one warp's share
+                     of the edges, 512 .. 4096) */
+  int chunk_min;  /* rows with more in-edges than this are cut into chunks (default 4096, or
+                     chunk's when both are 0) */
   int hot_entries;/* contributions of the highest in-degree vertices kept in shared memory
-                     by the persistent kernel, multiple of 4, <= 56832 (default 32768) */
+                     by the persistent kernel, multiple of 4, <= 56832 (default 32768; from
+                     2^19 edges up edges / 200, 4096 .. 32768) */
   int flags;      /* GPR_LAYOUT_* bits */
   int block_rows; /* blocked form: rows per block, <= 12288 (default: about rows / (2 SMs),
                      256 .. 12288) */

@@ -10,7 +10,7 @@ Tolerances (the bar this path is held to):
 import numpy as np
 import pytest
 
-from graphs import degree_ladder, erdos_renyi, star
+from graphs import degree_ladder, erdos_renyi, in_csr, star
 
 pytestmark = pytest.mark.gpu
 
@@ -295,3 +295,28 @@ def test_large_graph_solved_after_a_small_one_was_made(G, O, blocked):
             g2.pagerank(tol=0.0, max_iter=3, form=form)
             s, _ = g.pagerank(tol=0.0, max_iter=3, form=form)
     assert np.array_equal(s, ref)
+
+
+@pytest.mark.parametrize("deg", [6, 14, 30])
+def test_default_bins_by_size(G, O, deg):
+    # From 2^19 edges up the default chunks shrink to a warp's share (at least 512
+    # edges): rows on and around the chunk sizes, in one graph and in a batch,
+    # which gives each graph the bits of its own solve.
+    rng = np.random.default_rng(deg)
+    m = 36000
+    hubs = [511, 512, 513, 1024, 1025, 4096, 4097, 9000]
+    src = np.concatenate([rng.choice(m, d, replace=False) for d in hubs]
+                         + [rng.integers(0, m, deg * m)])
+    dst = np.concatenate([np.repeat(np.arange(len(hubs)), hubs), rng.integers(8, m, deg * m)])
+    rp, col, od = in_csr(m, src, dst)
+    s, st, _, lay = solve(G, rp, col, od, tol=0.0, max_iter=6)
+    assert lay["n_long"] == np.sum(np.diff(rp) > (4096 if len(col) < 1 << 19 else 512))
+    ref, _, _ = O.pr_plain_f32(rp, col, od, tol=0.0, max_iter=6)
+    s64, _, _ = O.pr_f64(rp, col, od, tol=0.0, max_iter=6)
+    assert np.all(np.abs(s - ref) <= ABS_TOL + np.abs(ref - s64))
+    rp2, col2, od2 = erdos_renyi(700, 5, seed=deg)
+    with G.MultiGraph(np.concatenate([rp, rp2[1:] + rp[-1]]), np.concatenate([col, col2 + m]),
+                      np.concatenate([od, od2]), np.array([0, m, m + 700])) as mg:
+        b, _, _, _ = mg.pagerank(tol=0.0, max_iter=6)
+    small, _, _, _ = solve(G, rp2, col2, od2, tol=0.0, max_iter=6)
+    assert np.array_equal(b[:m], s) and np.array_equal(b[m:], small)
