@@ -184,10 +184,18 @@ int validate_csr(int m, long long nnz, int ncols, const int *d_rowptr,
 int validate_cols(long long nnz, int ncols, const int *d_col, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
-// SpMV layout: natural row order.  Rows with more than sell_max entries are
-// long rows handled in chunks (listed in long_rows); every other row sits in
-// a SELL-32 slice with its own length (sell_len, 255 marks a long row whose
-// lane is idle in the slice).
+// SpMV layout.  Rows with more than sell_max entries are long rows handled in
+// chunks (listed in long_rows); every other row sits in a SELL-32 slice, one
+// lane per row, with its own length.
+//   even lengths   rows in natural order (x and y locality of a stencil):
+//                  lane l of slice s is row 32 s + l, sell_len[row] its
+//                  length (255: long row, the lane is idle)
+//   ragged         (natural slices would be padded by more than 1/8) rows
+//                  sorted by descending length inside windows of kSpmvWindow
+//                  rows: slot_row[slot] is the row (-1: none), sell_len[slot]
+//                  its length.  When enough entries fall on few columns, the
+//                  `hot` most frequent columns are listed in hot_col and an
+//                  entry of column hot_col[h] stores ~h instead of the column.
 // ---------------------------------------------------------------------------
 struct SpmvLayout {
   int m = 0;
@@ -203,14 +211,25 @@ struct SpmvLayout {
   long long *slice_ptr = nullptr;  // [n_slices+1]
   int *sell_col = nullptr;
   float *sell_val = nullptr;
-  unsigned char *sell_len = nullptr;  // [m]
+  unsigned char *sell_len = nullptr;  // [32 n_slices] (even: rows, ragged: slots)
+  bool ragged = false;
+  int *slot_row = nullptr;         // [32 n_slices], ragged only
+  int *slice_at = nullptr;         // [n_slices+1] slice_ptr / 32, ragged only
+  int4 *chunk_desc = nullptr;      // [n_chunks], ragged only: {row, first entry / 4, entries,
+                                   // index into long_rows or -1 when the row has one chunk}
+  int hot = 0;                     // columns staged in shared memory
+  int *hot_col = nullptr;          // [hot]
   long long long_elems = 0, sell_elems = 0;
   long long device_bytes = 0;
 };
 
+constexpr int kSpmvWindow = 1024;  // rows sorted together in a ragged layout
+constexpr int kSpmvHotMax = 16384;
+// hot_columns: look for columns to stage in shared memory (a histogram and a sort
+// of the columns; worth it for a matrix that is multiplied more than once).
 int build_spmv_layout(int m, long long nnz, const int *d_Ap, const int *d_Aj,
-                      const float *d_Ax, int sell_max, int chunk, SpmvLayout *L,
-                      cudaStream_t st);
+                      const float *d_Ax, int sell_max, int chunk, bool hot_columns,
+                      SpmvLayout *L, cudaStream_t st);
 void free_spmv_layout(SpmvLayout *L);
 
 }  // namespace gpr

@@ -6,6 +6,9 @@
 // small, cache-friendly prefix.  Edge order inside each row is preserved.
 #include <cub/cub.cuh>
 
+#include <algorithm>
+#include <vector>
+
 #include "gpr_internal.cuh"
 
 namespace gpr {
@@ -31,6 +34,11 @@ __global__ void k_validate_cols(long long nnz, int ncols, const int *__restrict_
     int c = col[e];
     if (c < 0 || c >= ncols) atomicOr(flag, 8);
   }
+}
+
+__global__ void k_iota(int m, int *iota) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < m) iota[i] = i;
 }
 
 __global__ void k_indeg_iota(int m, const int *__restrict__ rowptr, int *indeg, int *iota) {
@@ -417,10 +425,11 @@ void free_pr_layout(PrLayout *L) {
 }
 
 // ---------------------------------------------------------------------------
-// SpMV layout (natural row order)
+// SpMV layout
 // ---------------------------------------------------------------------------
 namespace {
 
+// Long rows (more than sell_max entries) flagged; the others' lengths.
 __global__ void k_spmv_flags(int m, const int *__restrict__ Ap, int sell_max, int *is_long,
                              unsigned char *sell_len) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -447,23 +456,44 @@ __global__ void k_spmv_long_lens(int n_long, const int *__restrict__ rows,
   }
 }
 
-__global__ void k_spmv_fill_long(int n_long, const int *__restrict__ rows,
+// An entry's stored column: ~h for a hot column (hot_at: h of each column or -1).
+__device__ __forceinline__ int spmv_col(const int *__restrict__ hot_at, int c) {
+  if (!hot_at) return c;
+  const int h = hot_at[c];
+  return h >= 0 ? ~h : c;
+}
+
+// One warp per chunk of a long row.
+__global__ void k_spmv_fill_long(int n_chunks, int chunk, const int *__restrict__ chunk_row,
+                                 const int *__restrict__ cbeg, const int *__restrict__ rows,
                                  const int *__restrict__ Ap, const int *__restrict__ Aj,
-                                 const float *__restrict__ Ax,
+                                 const float *__restrict__ Ax, const int *__restrict__ hot_at,
                                  const long long *__restrict__ lptr, int *lcol, float *lval) {
   int lane = threadIdx.x & 31;
   long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long i = w; i < n_long; i += nw) {
-    int r = rows[i];
-    long long sb = Ap[r], deg = Ap[r + 1] - sb;
-    long long db = lptr[i], plen = lptr[i + 1] - db;
-    for (long long k = lane; k < plen; k += 32) {
+  for (long long c = w; c < n_chunks; c += nw) {
+    const int i = chunk_row[c], r = rows[i];
+    const long long sb = Ap[r], deg = Ap[r + 1] - sb;
+    const long long db = lptr[i], plen = lptr[i + 1] - db;
+    const long long k0 = (c - cbeg[i]) * chunk, k1 = min(plen, k0 + chunk);
+    for (long long k = k0 + lane; k < k1; k += 32) {
       bool v = k < deg;
-      lcol[db + k] = v ? Aj[sb + k] : 0;
+      lcol[db + k] = v ? spmv_col(hot_at, Aj[sb + k]) : 0;
       lval[db + k] = v ? Ax[sb + k] : 0.0f;
     }
   }
+}
+
+__global__ void k_spmv_chunk_desc(int n_chunks, int chunk, const int *__restrict__ chunk_row,
+                                  const int *__restrict__ cbeg, const int *__restrict__ rows,
+                                  const long long *__restrict__ lptr, int4 *desc) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n_chunks) return;
+  const int i = chunk_row[c];
+  const long long b = lptr[i] + (long long)(c - cbeg[i]) * chunk;
+  const long long e = min(b + (long long)chunk, lptr[i + 1]);
+  desc[c] = make_int4(rows[i], (int)(b >> 2), (int)(e - b), cbeg[i + 1] - cbeg[i] == 1 ? -1 : i);
 }
 
 __global__ void k_spmv_slice_lens(int m, int n_slices, const unsigned char *__restrict__ len,
@@ -481,34 +511,124 @@ __global__ void k_spmv_slice_lens(int m, int n_slices, const unsigned char *__re
   }
 }
 
+// One CTA of kSpmvWindow threads per window: slot of each row by descending
+// length (long rows as 0), stable; slots past the last row are empty.
+__global__ void k_spmv_window(int m, const unsigned char *__restrict__ row_len, int *slot_row,
+                              unsigned char *slot_len) {
+  __shared__ __align__(4) unsigned char s_len[kSpmvWindow];
+  const long long r = (long long)blockIdx.x * kSpmvWindow + threadIdx.x;
+  int d = r < m ? row_len[r] : 0;
+  if (d == 255) d = 0;
+  s_len[threadIdx.x] = (unsigned char)d;
+  __syncthreads();
+  int rank = 0;
+  for (int i = 0; i < kSpmvWindow; ++i) {
+    const int o = s_len[i];
+    rank += (o > d || (o == d && i < (int)threadIdx.x)) ? 1 : 0;
+  }
+  const long long slot = (long long)blockIdx.x * kSpmvWindow + rank;
+  slot_row[slot] = r < m ? (int)r : -1;
+  slot_len[slot] = (unsigned char)d;
+}
+
 __global__ void k_spmv_fill_sell(int m, int n_slices, const int *__restrict__ Ap,
                                  const int *__restrict__ Aj, const float *__restrict__ Ax,
                                  const unsigned char *__restrict__ len,
+                                 const int *__restrict__ slot_row, const int *__restrict__ hot_at,
                                  const long long *__restrict__ sptr, int *scol, float *sval) {
   long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= 32LL * n_slices) return;
   int s = (int)(t >> 5), lane = (int)(t & 31);
   long long base = sptr[s];
   int slen = (int)((sptr[s + 1] - base) >> 5);
-  long long r = 32LL * s + lane;
+  const long long r = slot_row ? slot_row[t] : t;
   int d = 0;
   long long sb = 0;
-  if (r < m && len[r] != 255) {
-    d = len[r];
+  if (r >= 0 && r < m && len[t] != 255) {
+    d = len[t];
     sb = Ap[r];
   }
   for (int j = 0; j < slen; ++j) {
     bool v = j < d;
-    scol[base + 32LL * j + lane] = v ? Aj[sb + j] : 0;
+    scol[base + 32LL * j + lane] = v ? spmv_col(hot_at, Aj[sb + j]) : 0;
     sval[base + 32LL * j + lane] = v ? Ax[sb + j] : 0.0f;
   }
+}
+
+__global__ void k_slice_at(int n, const long long *__restrict__ sptr, int *at) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < n) at[s] = (int)(sptr[s] >> 5);
+}
+
+__global__ void k_col_count(long long nnz, const int *__restrict__ Aj, int *count) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nnz; e += stride)
+    atomicAdd(count + Aj[e], 1);
+}
+
+__global__ void k_hot_at(int hot, const int *__restrict__ hot_col, int *hot_at) {
+  const int h = blockIdx.x * blockDim.x + threadIdx.x;
+  if (h < hot) hot_at[hot_col[h]] = h;
+}
+
+// Columns to stage: the H most frequent ones, H the power of two whose staged
+// gathers, less the 148 H loads that staging costs (one CTA per SM), are most; none
+// unless that is over 1/16 of all entries.  *hot_at: H's index of each column.
+int find_hot_columns(int m, long long nnz, const int *d_Aj, SpmvLayout *L, int **hot_at,
+                     cudaStream_t st) {
+  Scratch S;
+  int *count = nullptr, *iota = nullptr, *scount = nullptr, *cols = nullptr;
+  GPR_TRY(dalloc(&count, m, "column counts"));
+  S.p[0] = count;
+  GPR_TRY(dalloc(&iota, m, "iota"));
+  S.p[1] = iota;
+  GPR_TRY(dalloc(&scount, m, "sorted counts"));
+  S.p[2] = scount;
+  GPR_TRY(dalloc(&cols, m, "sorted columns"));
+  S.p[3] = cols;
+  GPR_CUDA(cudaMemsetAsync(count, 0, sizeof(int) * (size_t)m, st));
+  k_col_count<<<std::min(grid_for(nnz), 148u * 32u), 256, 0, st>>>(nnz, d_Aj, count);
+  k_iota<<<grid_for(m), 256, 0, st>>>(m, iota);
+  size_t tb = 0;
+  GPR_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, count, scount, iota, cols, m, 0,
+                                                     32, st));
+  void *tmp = nullptr;
+  GPR_TRY(dmalloc(&tmp, tb, "sort scratch"));
+  S.p[4] = tmp;
+  GPR_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp, tb, count, scount, iota, cols, m, 0, 32,
+                                                     st));
+  const int top = std::min(m, kSpmvHotMax);
+  std::vector<int> h((size_t)top);
+  GPR_CUDA(cudaMemcpyAsync(h.data(), scount, sizeof(int) * (size_t)top, cudaMemcpyDeviceToHost, st));
+  GPR_CUDA(cudaStreamSynchronize(st));
+  long long sum = 0, best = nnz / 16;
+  int hot = 0;
+  for (int i = 0; i < top; ++i) {
+    sum += h[i];
+    const int n = i + 1;
+    if (n >= 1024 && (n & (n - 1)) == 0 && sum - 148LL * n > best) {
+      best = sum - 148LL * n;
+      hot = n;
+    }
+  }
+  if (hot == 0) return GPR_OK;
+  GPR_TRY(dalloc(&L->hot_col, hot, "hot columns"));
+  GPR_TRY(dalloc(hot_at, m, "hot column index"));
+  L->hot = hot;
+  GPR_CUDA(cudaMemcpyAsync(L->hot_col, cols, sizeof(int) * (size_t)hot, cudaMemcpyDeviceToDevice,
+                           st));
+  GPR_CUDA(cudaMemsetAsync(*hot_at, 0xff, sizeof(int) * (size_t)m, st));
+  k_hot_at<<<grid_for(hot), 256, 0, st>>>(hot, L->hot_col, *hot_at);
+  GPR_CUDA(cudaGetLastError());
+  GPR_CUDA(cudaStreamSynchronize(st));
+  return GPR_OK;
 }
 
 }  // namespace
 
 int build_spmv_layout(int m, long long nnz, const int *d_Ap, const int *d_Aj,
-                      const float *d_Ax, int sell_max, int chunk, SpmvLayout *L,
-                      cudaStream_t st) {
+                      const float *d_Ax, int sell_max, int chunk, bool hot_columns,
+                      SpmvLayout *L, cudaStream_t st) {
   *L = SpmvLayout();
   L->m = m;
   L->nnz = nnz;
@@ -516,7 +636,8 @@ int build_spmv_layout(int m, long long nnz, const int *d_Ap, const int *d_Aj,
   L->chunk = chunk;
   if (m <= 0) return GPR_OK;
   Scratch S;
-  int *is_long = nullptr, *iota = nullptr, *nsel = nullptr;
+  int *is_long = nullptr, *iota = nullptr, *nsel = nullptr, *hot_at = nullptr;
+  unsigned char *row_len = nullptr;
   GPR_TRY(dalloc(&is_long, m, "long flags"));
   S.p[0] = is_long;
   GPR_TRY(dalloc(&iota, m, "iota"));
@@ -547,37 +668,72 @@ int build_spmv_layout(int m, long long nnz, const int *d_Ap, const int *d_Aj,
       L->n_long, L->long_rows, d_Ap, chunk, L->long_ptr, L->row_cbeg);
   GPR_TRY(exclusive_scan(L->long_ptr, (long long)L->n_long + 1, st));
   GPR_TRY(exclusive_scan(L->row_cbeg, (long long)L->n_long + 1, st));
+  // Slices in natural order; ragged when they would be padded by more than 1/8.
+  L->n_slices = (int)ceil_div(m, 32);
+  GPR_TRY(dalloc(&L->slice_ptr, (size_t)ceil_div(m, kSpmvWindow) * (kSpmvWindow / 32) + 1,
+                 "slice offsets"));
+  k_spmv_slice_lens<<<grid_for((long long)L->n_slices + 1), 256, 0, st>>>(
+      m, L->n_slices, L->sell_len, L->slice_ptr);
+  GPR_TRY(exclusive_scan(L->slice_ptr, (long long)L->n_slices + 1, st));
+  long long long_nnz = 0;
+  GPR_CUDA(cudaMemcpyAsync(&L->sell_elems, L->slice_ptr + L->n_slices, sizeof(long long),
+                           cudaMemcpyDeviceToHost, st));
   GPR_CUDA(cudaMemcpyAsync(&L->long_elems, L->long_ptr + L->n_long, sizeof(long long),
                            cudaMemcpyDeviceToHost, st));
   GPR_CUDA(cudaMemcpyAsync(&L->n_chunks, L->row_cbeg + L->n_long, sizeof(int),
                            cudaMemcpyDeviceToHost, st));
   GPR_CUDA(cudaStreamSynchronize(st));
+  long_nnz = L->long_elems;  // padded to multiples of 4: an upper bound
+  const long long short_nnz = std::max(0LL, nnz - long_nnz);
+  L->ragged = m <= 0x7fffffff - kSpmvWindow &&
+              (L->sell_elems > short_nnz + short_nnz / 8 + 1024 || L->long_elems > nnz / 8);
+  if (L->ragged) {
+    const int windows = (int)ceil_div(m, kSpmvWindow);
+    L->n_slices = windows * (kSpmvWindow / 32);
+    row_len = L->sell_len;
+    S.p[3] = row_len;
+    L->sell_len = nullptr;
+    GPR_TRY(dalloc(&L->sell_len, 32LL * L->n_slices, "slot lengths"));
+    GPR_TRY(dalloc(&L->slot_row, 32LL * L->n_slices, "slot rows"));
+    k_spmv_window<<<windows, kSpmvWindow, 0, st>>>(m, row_len, L->slot_row, L->sell_len);
+    k_spmv_slice_lens<<<grid_for((long long)L->n_slices + 1), 256, 0, st>>>(
+        32 * L->n_slices, L->n_slices, L->sell_len, L->slice_ptr);
+    GPR_TRY(exclusive_scan(L->slice_ptr, (long long)L->n_slices + 1, st));
+    GPR_CUDA(cudaMemcpyAsync(&L->sell_elems, L->slice_ptr + L->n_slices, sizeof(long long),
+                             cudaMemcpyDeviceToHost, st));
+    GPR_CUDA(cudaStreamSynchronize(st));
+    GPR_TRY(dalloc(&L->slice_at, (size_t)L->n_slices + 1, "slice offsets"));
+    k_slice_at<<<grid_for((long long)L->n_slices + 1), 256, 0, st>>>(L->n_slices + 1, L->slice_ptr,
+                                                                     L->slice_at);
+    if (hot_columns) GPR_TRY(find_hot_columns(m, nnz, d_Aj, L, &hot_at, st));
+    S.p[4] = hot_at;
+  }
   GPR_TRY(dalloc(&L->long_col, (size_t)L->long_elems, "long cols"));
   GPR_TRY(dalloc(&L->long_val, (size_t)L->long_elems, "long vals"));
   GPR_TRY(dalloc(&L->chunk_row, (size_t)L->n_chunks, "chunk rows"));
   if (L->n_long > 0) {
-    unsigned g = grid_for(32LL * L->n_long);
-    if (g > 148u * 32u) g = 148u * 32u;
+    unsigned g = std::min(grid_for(32LL * L->n_long), 148u * 32u);
     k_fill_chunk_row<<<g, 256, 0, st>>>(L->n_long, L->row_cbeg, L->chunk_row);
-    k_spmv_fill_long<<<g, 256, 0, st>>>(L->n_long, L->long_rows, d_Ap, d_Aj, d_Ax,
-                                        L->long_ptr, L->long_col, L->long_val);
+    g = std::min(grid_for(32LL * L->n_chunks), 148u * 32u);
+    k_spmv_fill_long<<<g, 256, 0, st>>>(L->n_chunks, chunk, L->chunk_row, L->row_cbeg,
+                                        L->long_rows, d_Ap, d_Aj, d_Ax, hot_at, L->long_ptr,
+                                        L->long_col, L->long_val);
+    if (L->ragged) {
+      GPR_TRY(dalloc(&L->chunk_desc, (size_t)L->n_chunks, "chunk descriptors"));
+      k_spmv_chunk_desc<<<grid_for(L->n_chunks), 256, 0, st>>>(
+          L->n_chunks, chunk, L->chunk_row, L->row_cbeg, L->long_rows, L->long_ptr, L->chunk_desc);
+    }
   }
-  L->n_slices = (int)ceil_div(m, 32);
-  GPR_TRY(dalloc(&L->slice_ptr, (size_t)L->n_slices + 1, "slice offsets"));
-  k_spmv_slice_lens<<<grid_for((long long)L->n_slices + 1), 256, 0, st>>>(
-      m, L->n_slices, L->sell_len, L->slice_ptr);
-  GPR_TRY(exclusive_scan(L->slice_ptr, (long long)L->n_slices + 1, st));
-  GPR_CUDA(cudaMemcpyAsync(&L->sell_elems, L->slice_ptr + L->n_slices, sizeof(long long),
-                           cudaMemcpyDeviceToHost, st));
-  GPR_CUDA(cudaStreamSynchronize(st));
   GPR_TRY(dalloc(&L->sell_col, (size_t)L->sell_elems, "sell cols"));
   GPR_TRY(dalloc(&L->sell_val, (size_t)L->sell_elems, "sell vals"));
   k_spmv_fill_sell<<<grid_for(32LL * L->n_slices), 256, 0, st>>>(
-      m, L->n_slices, d_Ap, d_Aj, d_Ax, L->sell_len, L->slice_ptr, L->sell_col, L->sell_val);
+      m, L->n_slices, d_Ap, d_Aj, d_Ax, L->sell_len, L->slot_row, hot_at, L->slice_ptr,
+      L->sell_col, L->sell_val);
   GPR_CUDA(cudaGetLastError());
   GPR_CUDA(cudaStreamSynchronize(st));
   L->device_bytes = (long long)m * 5 + 8LL * (L->n_long + 1) * 2 + 8LL * L->long_elems +
-                    4LL * L->n_chunks + 8LL * (L->n_slices + 1) + 8LL * L->sell_elems;
+                    4LL * L->n_chunks + 8LL * (L->n_slices + 1) + 8LL * L->sell_elems +
+                    (L->ragged ? 128LL * L->n_slices + 16LL * L->n_chunks + 4LL * L->hot : 0);
   return GPR_OK;
 }
 
@@ -592,6 +748,10 @@ void free_spmv_layout(SpmvLayout *L) {
   dfree(L->sell_col);
   dfree(L->sell_val);
   dfree(L->sell_len);
+  dfree(L->slot_row);
+  dfree(L->slice_at);
+  dfree(L->chunk_desc);
+  dfree(L->hot_col);
   *L = SpmvLayout();
 }
 

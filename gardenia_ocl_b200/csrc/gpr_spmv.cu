@@ -1,14 +1,19 @@
 // CSR SpMV y <- y + A*x on B200 (src/spmv/omp_base.cc:8-32 semantics).
 //
-// Rows keep their natural order (x locality of stencil-like matrices is the
-// main asset).  Rows with at most sell_max entries live in SELL-32 slices,
+// Rows with at most sell_max entries live in SELL-32 slices,
 // one lane per row: the lane starts from y[r] and adds x[j]*Ax[jj] in CSR
 // order with explicitly rounded multiply and add, i.e. the same float
 // operations in the same order as the reference's loop, so those rows are
 // bit-identical to it.  Longer rows are split into chunks of `chunk` entries
 // (one warp per chunk, 128-bit loads) whose partial sums the last arriving
 // warp combines in a fixed order.
+//   k_spmv       even row lengths: rows in natural order (x locality of
+//                stencil-like matrices is the main asset), a warp per slice
+//   k_spmv_rag   ragged rows (a graph's adjacency): rows sorted by length in
+//                windows, the most frequent columns' x staged in shared memory
 #include <string.h>
+
+#include <algorithm>
 
 #include "gpr_internal.cuh"
 #include "gpr_guard.h"
@@ -30,6 +35,13 @@ constexpr unsigned kFull = 0xffffffffu;
 // indices and values, then gathers their x.  On the 27-point 128^3 stencil
 // 4 / 8 / 16 per round ran at 85% / 99% / 90% of the measured copy bandwidth.
 constexpr int kSpmvU = 8;
+// The same for a ragged layout, and 16-byte loads of columns and of values per lane and
+// round of a chunk: what 64 registers hold.  RMAT, 2,500,009 rows, 38M entries: 8 and
+// 2 189 us, 12 and 3 164 us; two CTAs per SM at 32 registers with 4 and 1 189 us, 768
+// threads with 16 and 4 202 us.
+constexpr int kRagBlock = 1024;
+constexpr int kRagU = 12;
+constexpr int kRagU4 = 3;
 
 struct SpArgs {
   int m, n_long, n_chunks, n_slices, chunk;
@@ -43,6 +55,11 @@ struct SpArgs {
   const int *sell_col;
   const float *sell_val;
   const unsigned char *sell_len;
+  const int *slot_row;     // ragged layout: see SpmvLayout
+  const int4 *chunk_desc;
+  const int *slice_at;
+  int hot;
+  const int *hot_col;
   const float *x;
   float *y;
   float *partial;
@@ -165,6 +182,166 @@ __global__ void __launch_bounds__(gpr::kBlock) k_spmv(SpArgs a) {
   }
 }
 
+// x of a stored column: ~h is the h-th staged column.
+struct HotX {
+  const float *x;
+  const float *s_x;
+  __device__ __forceinline__ float operator()(int c) const {
+    const float *p = c >= 0 ? x + c : s_x + ~c;
+    float v;
+    asm volatile("ld.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+  }
+};
+
+// Slice of unit t of the slices: the widest of every window first, then the second of
+// every window and so on (rows are sorted inside the windows), so that the CTAs'
+// last units are narrow.
+__device__ __forceinline__ int rag_slice_of(const SpArgs &a, int t) {
+  constexpr int per = gpr::kSpmvWindow / 32;
+  const int windows = a.n_slices / per;
+  return (t % windows) * per + t / windows;
+}
+
+// What a warp needs to know of a unit before it can load its entries; fetched one
+// unit ahead.  Chunk: its descriptor.  Slice: {this lane's row, first column of the
+// slice in lines of 32 entries, end, this lane's entries}.
+__device__ __forceinline__ int4 rag_peek(const SpArgs &a, int u, int lane) {
+  int4 d = make_int4(-1, 0, 0, 0);
+  if (u < a.n_chunks) {
+    asm volatile("ld.global.nc.v4.s32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(d.x), "=r"(d.y), "=r"(d.z), "=r"(d.w) : "l"(a.chunk_desc + u));
+  } else if (u < a.n_chunks + a.n_slices) {
+    const int s = rag_slice_of(a, u - a.n_chunks);
+    unsigned w;
+    asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(d.x) : "l"(a.slot_row + s * 32 + lane));
+    asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(d.y) : "l"(a.slice_at + s));
+    asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(d.z) : "l"(a.slice_at + s + 1));
+    asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(w) : "l"(a.sell_len + s * 32 + lane));
+    d.w = (int)w;
+  }
+  return d;
+}
+
+__device__ __forceinline__ void rag_slice(const SpArgs &a, const HotX &gx, int4 u, int lane,
+                                          uint64_t pol) {
+  const int width = u.z - u.y, r = u.x, d = u.w;
+  if (width == 0) return;
+  const int *pc = a.sell_col + 32LL * u.y + lane;
+  const float *pv = a.sell_val + 32LL * u.y + lane;
+  float acc = d > 0 ? a.y[r] : 0.f;
+  for (int j0 = 0; j0 < width; j0 += kRagU) {
+    int c[kRagU];
+    float v[kRagU], xv[kRagU];
+#pragma unroll
+    for (int q = 0; q < kRagU; ++q) {
+      c[q] = 0;
+      v[q] = 0.f;
+      if (j0 + q < d) {
+        c[q] = ld_s32(pc + 32 * (j0 + q), pol);
+        v[q] = ld_f32(pv + 32 * (j0 + q), pol);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kRagU; ++q) {
+      xv[q] = 0.f;
+      if (j0 + q < d) xv[q] = gx(c[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < kRagU; ++q)
+      if (j0 + q < d) acc = __fadd_rn(acc, __fmul_rn(xv[q], v[q]));
+  }
+  if (d > 0) a.y[r] = acc;
+}
+
+__device__ __forceinline__ void rag_chunk(const SpArgs &a, const HotX &gx, int c, int4 d,
+                                          int lane, uint64_t pol) {
+  const long long b = 4LL * d.y;
+  float acc = 0.f;
+  for (int k0 = 4 * lane; k0 < d.z; k0 += 128 * kRagU4) {
+    int4 q[kRagU4];
+    float4 v[kRagU4];
+#pragma unroll
+    for (int i = 0; i < kRagU4; ++i) {
+      const bool in = k0 + 128 * i < d.z;
+      q[i] = in ? ld_s32x4(a.long_col + b + k0 + 128 * i, pol) : make_int4(-1, -1, -1, -1);
+      v[i] = in ? ld_f32x4(a.long_val + b + k0 + 128 * i, pol) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float xv[4 * kRagU4];
+#pragma unroll
+    for (int i = 0; i < kRagU4; ++i) {
+      const bool in = k0 + 128 * i < d.z;
+      xv[4 * i + 0] = in ? gx(q[i].x) : 0.f;
+      xv[4 * i + 1] = in ? gx(q[i].y) : 0.f;
+      xv[4 * i + 2] = in ? gx(q[i].z) : 0.f;
+      xv[4 * i + 3] = in ? gx(q[i].w) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < kRagU4; ++i)
+      if (k0 + 128 * i < d.z)
+        acc += (xv[4 * i] * v[i].x + xv[4 * i + 1] * v[i].y) +
+               (xv[4 * i + 2] * v[i].z + xv[4 * i + 3] * v[i].w);
+  }
+  acc = warp_sum(acc);
+  if (d.w < 0) {
+    if (lane == 0) a.y[d.x] = a.y[d.x] + acc;
+    return;
+  }
+  const int cb = a.row_cbeg[d.w], nc = a.row_cbeg[d.w + 1] - cb;
+  int last = 0;
+  if (lane == 0) {
+    a.partial[c] = acc;
+    __threadfence();
+    last = atomicAdd(a.cnt + d.w, 1) == nc - 1;
+  }
+  last = __shfl_sync(kFull, last, 0);
+  if (!last) return;
+  __threadfence();
+  float t = 0.f;
+  for (int q = lane; q < nc; q += 32) t += __ldcg(a.partial + cb + q);
+  t = warp_sum(t);
+  if (lane == 0) {
+    atomicExch(a.cnt + d.w, 0);
+    a.y[d.x] = a.y[d.x] + t;
+  }
+}
+
+// Ragged matrices: one 1024-thread CTA per SM.  What bounds them is single x gathers
+// from L2 (at most about one per clock and SM) and their latency, so the x of the most
+// frequent columns is staged in shared memory first; the units (chunks, then slices
+// from wide to narrow) are dealt out to the CTAs and a CTA's warps take them from a
+// counter in shared memory, the next unit's descriptor in flight while they work.
+// RMAT, 2,500,009 rows, 38M entries, y = A x with y cleared: 233 us with rows in
+// natural order (the slices padded, 128 entries of a chunk in flight per warp), 132 us
+// this way (one clock of an SM per 1.0 entries); without staged columns 204 against
+// 189 us (8 entries per round), with 32768 instead of 16384 175 against 164 us.
+__global__ void __launch_bounds__(kRagBlock, 1) k_spmv_rag(SpArgs a) {
+  extern __shared__ float s_x[];
+  __shared__ int s_next;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t pol = evict_first_policy();
+  if (threadIdx.x == 0) s_next = kRagBlock / 32;
+  for (int h = threadIdx.x; h < a.hot; h += kRagBlock) s_x[h] = __ldg(a.x + __ldg(a.hot_col + h));
+  __syncthreads();
+  const HotX gx{a.x, s_x};
+  const int n = a.n_chunks + a.n_slices, G = gridDim.x, n_mine = (n + G - 1) / G;
+  auto unit = [&](int k) {
+    return k < n_mine ? k * G + ((k & 1) ? G - 1 - (int)blockIdx.x : (int)blockIdx.x) : n;
+  };
+  int u = unit(warp);
+  int4 d = rag_peek(a, u, lane);
+  while (u < n) {
+    int k = 0;
+    if (lane == 0) k = atomicAdd(&s_next, 1);
+    const int un = unit(__shfl_sync(kFull, k, 0));
+    const int4 dn = rag_peek(a, un, lane);
+    if (u < a.n_chunks) rag_chunk(a, gx, u, d, lane, pol);
+    else rag_slice(a, gx, d, lane, pol);
+    u = un;
+    d = dn;
+  }
+}
+
 void destroy(gpr_matrix *A) {
   if (!A) return;
   gpr::free_spmv_layout(&A->L);
@@ -174,7 +351,7 @@ void destroy(gpr_matrix *A) {
 }
 
 int create_impl(int m, long long nnz, const int *any_Ap, const int *any_Aj, const float *any_Ax,
-                gpr_matrix *A) {
+                bool hot_columns, gpr_matrix *A) {
   GPR_CUDA(cudaGetDevice(&A->device));
   cudaStream_t st = 0;
   void *ap = nullptr, *aj = nullptr, *ax = nullptr;
@@ -186,7 +363,7 @@ int create_impl(int m, long long nnz, const int *any_Ap, const int *any_Aj, cons
     rc = gpr::validate_csr(m, nnz, m, (const int *)ap, (const int *)aj, nullptr, st);
   if (rc == GPR_OK)
     rc = gpr::build_spmv_layout(m, nnz, (const int *)ap, (const int *)aj, (const float *)ax,
-                                gpr::kSellMaxDefault, gpr::kChunkDefault, &A->L, st);
+                                gpr::kSellMaxDefault, gpr::kChunkDefault, hot_columns, &A->L, st);
   cudaStreamSynchronize(st);
   if (oap) gpr::dfree(ap);
   if (oaj) gpr::dfree(aj);
@@ -196,6 +373,15 @@ int create_impl(int m, long long nnz, const int *any_Ap, const int *any_Aj, cons
   GPR_TRY(gpr::dalloc(&A->cnt, (size_t)A->L.n_long, "spmv counters"));
   GPR_CUDA(cudaMemset(A->cnt, 0, sizeof(int) * (A->L.n_long ? A->L.n_long : 1)));
   const long long units = (long long)A->L.n_chunks + A->L.n_slices;
+  if (A->L.ragged) {
+    int sms = 0;
+    GPR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, A->device));
+    GPR_CUDA(cudaFuncSetAttribute((const void *)k_spmv_rag,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(float) * gpr::kSpmvHotMax));
+    A->grid = (int)std::max<long long>(1, std::min<long long>(sms, gpr::ceil_div(units, 8)));
+    return GPR_OK;
+  }
   long long g = gpr::ceil_div(units, gpr::kBlock / 32);
   A->grid = (int)(g < 1 ? 1 : (g > 0x7fffffff ? 0x7fffffff : g));
   return GPR_OK;
@@ -203,11 +389,12 @@ int create_impl(int m, long long nnz, const int *any_Ap, const int *any_Aj, cons
 
 }  // namespace
 
-extern "C" {
+namespace {
 
-int gpr_matrix_create(int m, long long nnz, const int *any_Ap, const int *any_Aj,
-                      const float *any_Ax, gpr_matrix **out) {
-  GPR_ENTRY_BEGIN
+// hot_columns: a matrix that is multiplied more than once is worth the search for
+// the columns to stage; a one-shot call is not.
+int matrix_create(int m, long long nnz, const int *any_Ap, const int *any_Aj,
+                  const float *any_Ax, bool hot_columns, gpr_matrix **out) {
   if (!out) {
     gpr::set_error("gpr_matrix_create: NULL out");
     return GPR_EINVAL;
@@ -225,13 +412,23 @@ int gpr_matrix_create(int m, long long nnz, const int *any_Ap, const int *any_Aj
     return GPR_ENODEV;
   }
   gpr_matrix *A = new gpr_matrix();
-  int rc = create_impl(m, nnz, any_Ap, any_Aj, any_Ax, A);
+  int rc = create_impl(m, nnz, any_Ap, any_Aj, any_Ax, hot_columns, A);
   if (rc != GPR_OK) {
     destroy(A);
     return rc;
   }
   *out = A;
   return GPR_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int gpr_matrix_create(int m, long long nnz, const int *any_Ap, const int *any_Aj,
+                      const float *any_Ax, gpr_matrix **out) {
+  GPR_ENTRY_BEGIN
+  return matrix_create(m, nnz, any_Ap, any_Aj, any_Ax, true, out);
   GPR_ENTRY_END("gpr_matrix_create")
 }
 
@@ -267,7 +464,15 @@ int gpr_spmv(gpr_matrix *A, const float *d_x, float *d_y, void *stream) {
   a.y = d_y;
   a.partial = A->partial;
   a.cnt = A->cnt;
-  k_spmv<<<A->grid, gpr::kBlock, 0, (cudaStream_t)stream>>>(a);
+  a.slot_row = L.slot_row;
+  a.chunk_desc = L.chunk_desc;
+  a.slice_at = L.slice_at;
+  a.hot = L.hot;
+  a.hot_col = L.hot_col;
+  if (L.ragged)
+    k_spmv_rag<<<A->grid, kRagBlock, sizeof(float) * (size_t)L.hot, (cudaStream_t)stream>>>(a);
+  else
+    k_spmv<<<A->grid, gpr::kBlock, 0, (cudaStream_t)stream>>>(a);
   GPR_CUDA(cudaGetLastError());
   return GPR_OK;
 }
@@ -293,7 +498,7 @@ int gpr_spmv_solver(int m, int nnz, const int *Ap, const int *Aj, const float *A
     return GPR_EINVAL;
   }
   gpr_matrix *A = nullptr;
-  GPR_TRY(gpr_matrix_create(m, nnz, Ap, Aj, Ax, &A));
+  GPR_TRY(matrix_create(m, nnz, Ap, Aj, Ax, false, &A));
   void *dx = nullptr, *dy = nullptr;
   bool ox = false, oy = false;
   int rc = gpr::to_device(x, sizeof(float) * (size_t)m, &dx, &ox, 0, "x");

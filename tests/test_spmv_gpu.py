@@ -72,3 +72,39 @@ def test_empty_matrix(G):
     G.SpmvSolver(10, 0, Ap, np.array([], np.int32), np.array([], np.float32),
                  np.ones(10, np.float32), y)
     assert np.array_equal(y, np.arange(10, dtype=np.float32))
+
+
+@pytest.mark.parametrize("m", [1, 1023, 1024, 1025, 40000])
+@pytest.mark.parametrize("hot", [False, True])
+def test_ragged_matrix(G, O, m, hot):
+    """Ragged row lengths (windows of 1024 rows sorted by length), a matrix smaller than
+    a window and one row short of and past it, frequent columns staged in shared
+    memory or none frequent; empty rows, lengths around a lane's row (64), a
+    chunk's round (384) and a chunk (4096).  Short rows are the oracle's bits."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(m + hot)
+    lens = np.minimum(rng.zipf(1.6, m) - 1, 60)
+    edge = [63, 64, 65, 383, 384, 385, 4095, 4096, 4097, 9000, 0, 1, 12, 13]
+    for i, d in enumerate(edge):
+        if i < m:
+            lens[(i * 71) % m] = d
+    Ap = np.zeros(m + 1, np.int32)
+    np.cumsum(lens, out=Ap[1:])
+    n = int(Ap[-1])
+    Aj = (m * rng.random(n) ** (6 if hot else 1)).astype(np.int32)
+    Ax = rng.standard_normal(n).astype(np.float32)
+    x = rng.standard_normal(m).astype(np.float32)
+    y0 = rng.standard_normal(m).astype(np.float32)
+    ref = O.spmv_f32(Ap, Aj, Ax, x, y0)
+    A = G.Matrix(Ap, Aj, Ax)
+    dx, y = torch.from_numpy(x).cuda(), torch.from_numpy(y0.copy()).cuda()
+    A.spmv(dx, y, torch.cuda.current_stream().cuda_stream)
+    got = y.cpu().numpy()
+    A.close()
+    once = y0.copy()
+    G.SpmvSolver(m, n, Ap, Aj, Ax, x, once)
+    absum = np.abs(y0).astype(np.float64)
+    np.add.at(absum, np.repeat(np.arange(m), lens), np.abs(x[Aj] * Ax))
+    for out in (got, once):
+        assert np.array_equal(out[lens <= 64], ref[lens <= 64])
+        assert np.all(np.abs(out - ref) <= 1e-6 * absum + 1e-30)
