@@ -23,9 +23,9 @@ int dalloc(T **p, size_t count, const char *what) {
 void dfree(void *p);
 
 // While an instance lives, dfree on this thread only records the pointers;
-// the destructor frees them.  A free synchronises the device (cudaFree, or
-// the block cache's wait before reuse), so code that overlaps a copy on one
-// stream with work on another holds one until both streams are done.
+// the destructor frees them.  A freed block is handed out again behind a device
+// synchronisation, so code that overlaps a copy on one stream with work on another
+// holds one until both streams are done.
 class DeferFrees {
  public:
   DeferFrees();

@@ -398,12 +398,13 @@ int gpr_gen_stencil27(int n, int **d_Ap, int **d_Aj, float **d_Ax,
 /* Seeded uniform [0,1) floats (24 random bits). */
 int gpr_gen_uniform(long long n, unsigned long long seed, float *d_out);
 int gpr_free(void *d_ptr);
-/* The library keeps device blocks of 1 MiB and more after they are freed
- * (at most 24 GiB, reused by later requests that fit them within 1/8), so
- * one-shot calls do not map and unmap gigabytes each time.  Freeing a block
- * synchronises the device first, as cudaFree does.  gpr_release_cached returns
- * every cached block to the CUDA driver (released_bytes may be NULL);
- * gpr_cached_bytes reports how much is held. */
+/* The library keeps device blocks after they are freed: of 1 MiB and more at most
+ * 24 GiB, reused by later requests that fit them within 1/8; smaller ones, in powers
+ * of two, at most 64 MiB.  One-shot calls then do not map and unmap gigabytes each
+ * time nor wait for the device at every small free; a kept block is handed out
+ * again behind a device synchronisation.  gpr_free synchronises the device first, as
+ * cudaFree does.  gpr_release_cached returns every cached block to the CUDA driver
+ * (released_bytes may be NULL); gpr_cached_bytes reports how much is held. */
 int gpr_release_cached(long long *released_bytes);
 int gpr_cached_bytes(long long *bytes);
 /* Device allocation / copy helpers for callers without a CUDA runtime of

@@ -168,3 +168,27 @@ def test_block_cache_reuses_and_releases(G):
     assert q.value == first
     assert G.lib().gpr_free(q) == 0
     assert G.release_cached() >= 64 << 20 and G.cached_bytes() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("size", [1, 512, 513, 300000, 524288, 524289, (1 << 20) - 1, 1 << 20])
+def test_small_blocks_are_kept_by_size_class(G, size):
+    """A freed block comes back for the next request of its size class and holds what is
+    written to it; release returns all of them."""
+    G.release_cached()
+    p, q, r = C.c_void_p(), C.c_void_p(), C.c_void_p()
+    assert G.lib().gpr_malloc(C.byref(p), size) == 0
+    assert G.lib().gpr_malloc(C.byref(q), size) == 0
+    assert p.value != q.value
+    first = q.value
+    assert G.lib().gpr_free(q) == 0
+    assert G.cached_bytes() >= size
+    assert G.lib().gpr_malloc(C.byref(r), size) == 0
+    assert r.value == first
+    a = np.arange(size, dtype=np.int64).astype(np.uint8)
+    b = np.zeros_like(a)
+    for d, s in ((r, C.c_void_p(a.ctypes.data)), (C.c_void_p(b.ctypes.data), r)):
+        assert G.lib().gpr_memcpy(d, s, size) == 0
+    assert np.array_equal(a, b)
+    assert G.lib().gpr_free(p) == 0 and G.lib().gpr_free(r) == 0
+    assert G.release_cached() >= 2 * size and G.cached_bytes() == 0
