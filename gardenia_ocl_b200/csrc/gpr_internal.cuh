@@ -273,7 +273,8 @@ struct gpr_graph {
   double *cta_err = nullptr; // [2 * max grid] per-CTA residual partials
   double *err_hist = nullptr;// [err_cap] residual of every sweep
   unsigned *bar = nullptr;   // [4] grid barrier: arrivals, generation
-  int *status = nullptr;     // [4] error flags, sweeps done, done flag
+  int *status = nullptr;     // [8] error flags, sweeps done, done flag, launches, last
+                             // residual (double)
   float *scores_tmp = nullptr; // [m] device copy of host scores
   double *res_tmp = nullptr;   // [m+1+n_long] FP64 residual scratch
   int err_cap = 0;

@@ -335,6 +335,7 @@ __global__ void __launch_bounds__(1024, MINB) k_pr_hot(PrArgs a) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.status[1] = it;
     a.status[2] = 1;
+    *reinterpret_cast<double *>(a.status + 4) = s_total;  // of the last sweep
   }
 }
 
@@ -410,6 +411,7 @@ __global__ void __launch_bounds__(NT, MINB) k_pr_blocked(PrArgs a) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.status[1] = it;
     a.status[2] = 1;
+    *reinterpret_cast<double *>(a.status + 4) = s_total;  // of the last sweep
   }
 }
 
@@ -483,11 +485,37 @@ __global__ void __launch_bounds__(gpr::kBlock) k_pr_step(PrArgs a) {
   }
 }
 
-// Scores into the relabelled order and the first sweep's contributions.
+// The words that a solve starts from zero: barrier, status, queue heads, arrival
+// counters of multi-chunk rows and of multi-tile blocks, largest score.
+struct PrZero {
+  unsigned *bar;    // [4]
+  int *status;      // [8]
+  int *wq;          // [2]
+  int *cnt;         // [n_cnt]
+  int *bcnt;        // [n_bcnt]
+  int *tq;          // [2] (null: exact order)
+  unsigned *fx_max; // [1]
+  int n_cnt, n_bcnt;
+};
+
+// Scores into the relabelled order, the first sweep's contributions, and the words
+// above (a launch instead of six small memsets).
 template <typename T>
 __global__ void k_pr_prologue(int m, const int *__restrict__ perm, const int *__restrict__ outdeg,
-                              const float *__restrict__ scores_in, float *s, T *c0, T *c1) {
+                              const float *__restrict__ scores_in, float *s, T *c0, T *c1,
+                              PrZero z) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < z.n_cnt) z.cnt[i] = 0;
+  if (i < z.n_bcnt) z.bcnt[i] = 0;
+  if (i < 8) {
+    z.status[i] = 0;
+    if (i < 4) z.bar[i] = 0u;
+    if (i < 2) z.wq[i] = 0;
+    if (z.tq) {
+      if (i < 2) z.tq[i] = 0;
+      if (i < 1) z.fx_max[i] = 0u;
+    }
+  }
   if (i < m) {
     const float v = scores_in[perm[i]];
     s[i] = v;
@@ -841,7 +869,7 @@ int create_impl(int m, long long nnz, const int *any_rowptr, const int *any_col,
   GPR_TRY(gpr::dalloc(&g->partial, (size_t)L.n_chunks, "chunk partials"));
   GPR_TRY(gpr::dalloc(&g->cnt, (size_t)L.n_long, "chunk counters"));
   GPR_TRY(gpr::dalloc(&g->bar, 4, "barrier"));
-  GPR_TRY(gpr::dalloc(&g->status, 4, "status"));
+  GPR_TRY(gpr::dalloc(&g->status, 8, "status"));
   GPR_TRY(gpr::dalloc(&g->scores_tmp, (size_t)m, "score staging"));
   GPR_CUDA(cudaMemsetAsync(g->cnt, 0, sizeof(int) * (L.n_long ? L.n_long : 1), st));
 
@@ -960,20 +988,17 @@ int solve_impl(gpr_graph *g, float *d_scores, const gpr_pr_opts &o, int ki, gpr_
     GPR_CUDA(cudaMemsetAsync(g->h0, 0, 2 * cnh, st));
     GPR_CUDA(cudaMemsetAsync(g->h1, 0, 2 * cnh, st));
   }
-  GPR_CUDA(cudaMemsetAsync(g->bar, 0, 4 * sizeof(unsigned), st));
-  GPR_CUDA(cudaMemsetAsync(g->status, 0, 4 * sizeof(int), st));
-  GPR_CUDA(cudaMemsetAsync(g->wq, 0, 2 * sizeof(int), st));
-  if (g->L.n_long) GPR_CUDA(cudaMemsetAsync(g->cnt, 0, sizeof(int) * g->L.n_long, st));
   const gpr::BlockedLayout &B = g->B;
+  PrZero z = {g->bar, g->status, g->wq, g->cnt, nullptr, nullptr, nullptr, g->L.n_long, 0};
   if (blocked) {
-    GPR_CUDA(cudaMemsetAsync(g->tq, 0, 2 * sizeof(int), st));
-    GPR_CUDA(cudaMemsetAsync(g->fx_max, 0, sizeof(unsigned), st));
-    if (B.n_blocks) {
-      // clean after an abandoned solve; a completed sweep leaves them clean
-      GPR_CUDA(cudaMemsetAsync(B.bcnt, 0, sizeof(int) * B.n_blocks, st));
-      GPR_CUDA(cudaMemsetAsync(B.gacc, 0, 8 * (size_t)B.gacc_rows, st));
-    }
+    z.tq = g->tq;
+    z.fx_max = g->fx_max;
+    z.bcnt = B.bcnt;
+    z.n_bcnt = B.n_blocks;
+    // clean after an abandoned solve; a completed sweep leaves them clean
+    if (B.n_blocks) GPR_CUDA(cudaMemsetAsync(B.gacc, 0, 8 * (size_t)B.gacc_rows, st));
   }
+  const long long n_pro = std::max<long long>((long long)m + 1, std::max(8, std::max(z.n_cnt, z.n_bcnt)));
   PrArgs a = make_args(g, o, ki);
   if (blocked) {
     a.n_tiles = B.n_tiles;
@@ -998,12 +1023,12 @@ int solve_impl(gpr_graph *g, float *d_scores, const gpr_pr_opts &o, int ki, gpr_
   bool graph_mode = false;
   GPR_CUDA(cudaEventRecord(g->e0, st));
   if (kKernels[ki].elem == 2)
-    k_pr_prologue<bf16><<<grid_for((long long)m + 1), 256, 0, st>>>(
+    k_pr_prologue<bf16><<<grid_for(n_pro), 256, 0, st>>>(
         m, g->L.perm, g->L.outdeg, d_scores, g->s, static_cast<bf16 *>(g->h0),
-        static_cast<bf16 *>(g->h1));
+        static_cast<bf16 *>(g->h1), z);
   else
-    k_pr_prologue<float><<<grid_for((long long)m + 1), 256, 0, st>>>(
-        m, g->L.perm, g->L.outdeg, d_scores, g->s, g->c0, g->c1);
+    k_pr_prologue<float><<<grid_for(n_pro), 256, 0, st>>>(
+        m, g->L.perm, g->L.outdeg, d_scores, g->s, g->c0, g->c1, z);
   ++launches;
   if (blocked) {
     k_max_abs<<<std::min<unsigned>(grid_for(m), 148 * 8), 256, 0, st>>>(m, g->s, g->fx_max);
@@ -1068,7 +1093,7 @@ int solve_impl(gpr_graph *g, float *d_scores, const gpr_pr_opts &o, int ki, gpr_
   ++launches;
   GPR_CUDA(cudaGetLastError());
   GPR_CUDA(cudaEventRecord(g->e1, st));
-  int hs[4];
+  int hs[8];  // status, then the persistent kernels' last residual
   GPR_CUDA(cudaMemcpyAsync(hs, g->status, sizeof(hs), cudaMemcpyDeviceToHost, st));
   GPR_CUDA(cudaStreamSynchronize(st));
   float ms = 0.f, lms = 0.f;
@@ -1080,9 +1105,11 @@ int solve_impl(gpr_graph *g, float *d_scores, const gpr_pr_opts &o, int ki, gpr_
   g->last_sweeps = hs[1];
   out->solve_ms = ms;
   out->gpu_launches = launches + (graph_mode ? hs[1] : 0);
-  if (hs[1] > 0)
+  if (hs[1] > 0 && graph_mode)
     GPR_CUDA(cudaMemcpy(&out->residual, g->err_hist + hs[1] - 1, sizeof(double),
                         cudaMemcpyDeviceToHost));
+  else if (hs[1] > 0)
+    memcpy(&out->residual, hs + 4, sizeof(double));
   if (hs[0] & 1) {
     gpr::set_error("grid barrier wait exceeded %.3f s (sweep loop abandoned)", o.timeout_s);
     return GPR_ETIMEOUT;
