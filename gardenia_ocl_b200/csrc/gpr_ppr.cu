@@ -42,6 +42,8 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kPprBlock = 256;
+constexpr long long kNzBits = 1LL << 20;  // most bits of the sparse sweeps' map
+constexpr int kSparseSweeps = 2;          // first sweeps of a solve that are sparse
 
 struct PprArgs {
   int m, n_long, n_nz, n_chunks, k, n_pk;
@@ -66,6 +68,11 @@ struct PprArgs {
   float damp;
   double tol;
   int max_iter, bar_expect;
+  int it0;               // first sweep (sparse kernel: 0)
+  // Sparse kernel: bit v >> nz_shift is set when vertex v may hold an x or a
+  // contribution that is not 0 (see k_ppr).
+  unsigned *nz;
+  int nz_shift;
   int repack_below;      // > 0: stop once at most this many vectors are still updating
   long long timeout_ns;
   unsigned long long cond;  // graph mode: while-node condition handle (0: none)
@@ -146,13 +153,26 @@ __device__ __forceinline__ bool is_active(const unsigned (&act)[4], int q) {
   return (act[q >> 5] >> (q & 31)) & 1u;
 }
 
+__device__ __forceinline__ bool nz_test(const PprArgs &a, int v) {
+  const int g = v >> a.nz_shift;
+  unsigned w;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(w) : "l"(a.nz + (g >> 5)));
+  return (w >> (g & 31)) & 1u;
+}
+
+__device__ __forceinline__ void nz_mark(const PprArgs &a, int v) {
+  if (nz_test(a, v)) return;
+  const int g = v >> a.nz_shift;
+  atomicOr(a.nz + (g >> 5), 1u << (g & 31));
+}
+
 // Sums in-neighbour rows over `niter` rounds; niter is warp-uniform.  In
 // round j this lane's sub-group covers edges [first + j*stride, +E) clipped
 // to `end`: lane lq holds the indices of edges lq + p*L (p < P), the
 // sub-group broadcasts them, and every lane gathers its C components of each
 // row.  Edges past the sub-group's end (or lanes with no live component)
 // gather the zero sentinel row, so every shuffle runs on the full warp.
-template <int K, typename T>
+template <int K, typename T, bool SP>
 __device__ __forceinline__ void gather_edges(const PprArgs &a, const T *cin, long long first,
                                              long long end, long long stride, int niter, int lq,
                                              bool live, float (&acc)[Shape<K>::C]) {
@@ -171,6 +191,15 @@ __device__ __forceinline__ void gather_edges(const PprArgs &a, const T *cin, lon
       // next round's indices are in flight while this round gathers
       const long long en = eb + stride + lq + p * L;
       nxt[p] = (j + 1 < niter && en < end) ? ld_idx(a.csr_col + en) : a.m;
+    }
+    if constexpr (SP) {  // sources whose contributions are all 0: the sentinel's row instead
+#pragma unroll
+      for (int p = 0; p < P; ++p)
+        if (my[p] != a.m && !nz_test(a, my[p])) my[p] = a.m;
+      bool some = false;
+#pragma unroll
+      for (int p = 0; p < P; ++p) some |= my[p] != a.m;
+      if (!__any_sync(kFull, some)) continue;
     }
     const int ng = (int)max(0LL, min((long long)E, end - eb));
     const int nmax = (int)__reduce_max_sync(kFull, (unsigned)ng);
@@ -224,7 +253,7 @@ __device__ __forceinline__ void row_fetch(const PprArgs &a, int v, int lq, int &
 
 // Update of row v from its pulled sums (acc) for this lane's components;
 // od and xo from row_fetch, sd the lane's seed vertices.
-template <int K, typename T>
+template <int K, typename T, bool SP>
 __device__ __forceinline__ void row_update(const PprArgs &a, T *cout, int v, int lq,
                                            const unsigned (&act)[4], const double *dang_cur,
                                            const int (&sd)[Shape<K>::C],
@@ -233,6 +262,7 @@ __device__ __forceinline__ void row_update(const PprArgs &a, T *cout, int v, int
                                            double (&err)[Shape<K>::C], double (&dng)[Shape<K>::C]) {
   constexpr int C = Shape<K>::C;
   const float inv = od > 0 ? 1.0f / (float)od : 0.f;
+  bool any = false;
 #pragma unroll
   for (int c = 0; c < C; ++c) {
     const int q = lq * C + c;
@@ -244,13 +274,15 @@ __device__ __forceinline__ void row_update(const PprArgs &a, T *cout, int v, int
     err[c] += fabs((double)xn - (double)xo[c]);
     store_c(cout + o, od > 0 ? xn * inv : 0.f);
     if (od == 0) dng[c] += (double)xn;
+    if (SP) any |= xn != 0.f;
   }
+  if (SP && any) nz_mark(a, v);
 }
 
 // One sweep of this CTA's share: packets of units, the seed rows without
 // in-edges, and the CTA's residual and dangling sums (per vector, warps in
 // order) into cta_red.  Ends with the CTA synchronised.
-template <int K, typename T>
+template <int K, typename T, bool SP>
 __device__ __forceinline__ void ppr_sweep(const PprArgs &a, int it, const int (&sd)[Shape<K>::C],
                                           double *s_red) {
   constexpr int L = Shape<K>::L, R = Shape<K>::R, C = Shape<K>::C, E = Shape<K>::E;
@@ -260,6 +292,16 @@ __device__ __forceinline__ void ppr_sweep(const PprArgs &a, int it, const int (&
   const T *cin = reinterpret_cast<const T *>((it & 1) ? a.c1 : a.c0);
   T *cout = reinterpret_cast<T *>((it & 1) ? a.c0 : a.c1);
   const double *dang_cur = a.dang + (it & 1) * K;
+  constexpr bool early = Shape<K>::early && !SP;
+  // whether this lane's part of row v can change: sparse sweeps leave rows alone that
+  // are 0 and stay 0
+  auto moves = [&](int v, const float (&acc)[C]) {
+    if (!SP) return true;
+    bool m = nz_test(a, v);
+#pragma unroll
+    for (int c = 0; c < C; ++c) m |= acc[c] != 0.f || sd[c] == v;
+    return m;
+  };
   unsigned act[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) act[i] = __ldcg(a.active + (it & 1) * 4 + i);
@@ -286,17 +328,19 @@ __device__ __forceinline__ void ppr_sweep(const PprArgs &a, int it, const int (&
       const int4 d = __ldg(a.cdesc + u);
       const int r = d.x, cb = d.w;
       const long long b = d.y, e = d.z;
-      if (Shape<K>::early && cb < 0) row_fetch<K>(a, r, lq, od, xo);  // the row's only chunk
+      if (early && cb < 0) row_fetch<K>(a, r, lq, od, xo);  // the row's only chunk
       const int niter = (int)gpr::ceil_div(e - b, (long long)R * E);
-      gather_edges<K, T>(a, cin, b + (long long)g * E, e, (long long)R * E, niter, lq, live,
+      gather_edges<K, T, SP>(a, cin, b + (long long)g * E, e, (long long)R * E, niter, lq, live,
                          acc);
 #pragma unroll
       for (int o = L; o < 32; o <<= 1)
 #pragma unroll
         for (int c = 0; c < C; ++c) acc[c] += __shfl_xor_sync(kFull, acc[c], o);
       if (cb < 0) {
-        if (!Shape<K>::early) row_fetch<K>(a, r, lq, od, xo);
-        if (g == 0) row_update<K, T>(a, cout, r, lq, act, dang_cur, sd, acc, od, xo, err, dng);
+        const bool upd = moves(r, acc);
+        if (!early && upd) row_fetch<K>(a, r, lq, od, xo);
+        if (g == 0 && upd)
+          row_update<K, T, SP>(a, cout, r, lq, act, dang_cur, sd, acc, od, xo, err, dng);
         continue;
       }
       if (g == 0)
@@ -311,14 +355,17 @@ __device__ __forceinline__ void ppr_sweep(const PprArgs &a, int it, const int (&
       if (!last) continue;
       __threadfence();
       // Sum the row's chunk partials in chunk order (sub-group 0).
-      row_fetch<K>(a, r, lq, od, xo);
+      if (!SP) row_fetch<K>(a, r, lq, od, xo);
 #pragma unroll
       for (int c = 0; c < C; ++c) acc[c] = 0.f;
       for (int q = 0; q < nc; ++q)
 #pragma unroll
         for (int c = 0; c < C; ++c) acc[c] += __ldcg(a.partial + (size_t)(cb + q) * K + lq * C + c);
       if (lane == 0) atomicExch(a.cnt + r, 0);
-      if (g == 0) row_update<K, T>(a, cout, r, lq, act, dang_cur, sd, acc, od, xo, err, dng);
+      const bool upd = moves(r, acc);
+      if (SP && upd) row_fetch<K>(a, r, lq, od, xo);
+      if (g == 0 && upd)
+        row_update<K, T, SP>(a, cout, r, lq, act, dang_cur, sd, acc, od, xo, err, dng);
     }
     if (u >= u1) continue;
     // Row groups; with the early fetch, the next group's row offsets are
@@ -348,17 +395,18 @@ __device__ __forceinline__ void ppr_sweep(const PprArgs &a, int it, const int (&
       int od = 0;
 #pragma unroll
       for (int c = 0; c < C; ++c) acc[c] = 0.f;
-      if (Shape<K>::early && has) row_fetch<K>(a, v, lq, od, xo);
+      if (early && has) row_fetch<K>(a, v, lq, od, xo);
       // Rows of one warp have nearly equal degrees (degree order); the
       // sub-groups loop to the warp's longest row.
       long long span = e1 - e0;
 #pragma unroll
       for (int o = L; o < 32; o <<= 1) span = max(span, __shfl_xor_sync(kFull, span, o));
-      gather_edges<K, T>(a, cin, e0, e1, (long long)E, (int)gpr::ceil_div(span, E), lq,
+      gather_edges<K, T, SP>(a, cin, e0, e1, (long long)E, (int)gpr::ceil_div(span, E), lq,
                          live && has, acc);
       // edges past this row's end gathered the sentinel row (zeros)
-      if (!Shape<K>::early && has) row_fetch<K>(a, v, lq, od, xo);
-      if (has) row_update<K, T>(a, cout, v, lq, act, dang_cur, sd, acc, od, xo, err, dng);
+      const bool upd = has && moves(v, acc);
+      if (!early && upd) row_fetch<K>(a, v, lq, od, xo);
+      if (upd) row_update<K, T, SP>(a, cout, v, lq, act, dang_cur, sd, acc, od, xo, err, dng);
     }
   }
   // Seed rows without in-edges: only their teleport term changes.
@@ -373,6 +421,7 @@ __device__ __forceinline__ void ppr_sweep(const PprArgs &a, int it, const int (&
       const int od = a.outdeg[v];
       a.x[o] = xn;
       store_c(cout + o, od > 0 ? xn * (1.0f / (float)od) : 0.f);
+      if (SP) nz_mark(a, v);
       se = fabs((double)xn - (double)xo);
       if (od == 0) sd = (double)xn;
     }
@@ -408,32 +457,70 @@ __device__ __forceinline__ void ppr_sweep(const PprArgs &a, int it, const int (&
 
 // Closes sweep it; run by all threads of the last CTA to finish the sweep,
 // after every CTA's cta_red and seed_red are visible.  Sums each vector's
-// residual and dangling mass over CTAs in CTA order (deterministic), records
+// residual and dangling mass over CTAs in a fixed order (deterministic), records
 // the residual and sweep count of the vectors that updated, freezes those
 // below tol, publishes the next sweep's masks and dangling mass, sets
 // status[2] to whether any vector keeps updating and resets the queue head
 // that sweep it + 2 reuses.
+//
+// Thread t adds vector t % K over the CTAs t / K, t / K + J, ... (J = threads /
+// K): neighbouring threads read neighbouring vectors, eight CTAs' values are
+// in flight per thread, and the J parts of a vector are then added in order.
+// (One thread per vector walking over all CTAs: RMAT s22 k = 8 6.71 ms per call
+// against 6.52, 1,000,003 vertices k = 100 12.81 against 12.36.)
 template <int K>
-__device__ __forceinline__ void ppr_close(const PprArgs &a, int it, unsigned *s_act) {
+__device__ __forceinline__ void ppr_close(const PprArgs &a, int it, unsigned *s_act,
+                                          double *s_red) {
+  constexpr int J = kPprBlock / K;
   const int G = gridDim.x;
   const double *dang_cur = a.dang + (it & 1) * K;
   unsigned act[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) act[i] = __ldcg(a.active + (it & 1) * 4 + i);
   if (threadIdx.x < 4) s_act[threadIdx.x] = act[threadIdx.x];
-  __syncthreads();
-  for (int q = threadIdx.x; q < K; q += blockDim.x) {
-    double te = __ldcg(a.seed_red + q), td = __ldcg(a.seed_red + K + q);
-    for (int c = 0; c < G; ++c) {
-      te += __ldcg(a.cta_red + (size_t)c * K + q);
-      td += __ldcg(a.cta_red + (size_t)(G + c) * K + q);
+  const int q = threadIdx.x % K, j = threadIdx.x / K;
+  double te = 0.0, td = 0.0;
+  for (int c = j; c < G; c += 8 * J) {
+    double e[8], d[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const bool in = c + i * J < G;
+      e[i] = in ? __ldcg(a.cta_red + (size_t)(c + i * J) * K + q) : 0.0;
+      d[i] = in ? __ldcg(a.cta_red + (size_t)(G + c + i * J) * K + q) : 0.0;
     }
-    a.res_hist[(size_t)it * K + q] = te;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      te += e[i];
+      td += d[i];
+    }
+  }
+  // lanes of a warp that hold the same vector (K < 32), then the parts in order
+#pragma unroll
+  for (int o = K; o < 32; o <<= 1) {
+    te += __shfl_xor_sync(kFull, te, o);
+    td += __shfl_xor_sync(kFull, td, o);
+  }
+  constexpr int P = K < 32 ? kPprBlock / 32 : J;  // parts of a vector
+  __syncthreads();
+  if (K >= 32 || (threadIdx.x & 31) < K) {
+    const int p = K < 32 ? threadIdx.x >> 5 : j;
+    s_red[p * K + q] = te;
+    s_red[(P + p) * K + q] = td;
+  }
+  __syncthreads();
+  if (threadIdx.x < K) {
+    double re = __ldcg(a.seed_red + q), rd = __ldcg(a.seed_red + K + q);
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      re += s_red[p * K + q];
+      rd += s_red[(P + p) * K + q];
+    }
+    a.res_hist[(size_t)it * K + q] = re;
     const bool was = is_active(act, q);
-    a.dang[((it + 1) & 1) * K + q] = was ? td : dang_cur[q];
+    a.dang[((it + 1) & 1) * K + q] = was ? rd : dang_cur[q];
     if (was) {
       a.iters[q] = it + 1;
-      if (te < a.tol) atomicAnd(&s_act[q >> 5], ~(1u << (q & 31)));
+      if (re < a.tol) atomicAnd(&s_act[q >> 5], ~(1u << (q & 31)));
     }
   }
   __syncthreads();
@@ -456,18 +543,31 @@ __device__ __forceinline__ void ppr_close(const PprArgs &a, int it, unsigned *s_
 // spills (+4% at K = 8); for wider vectors inlining is faster (-18% at
 // K = 128 as a call).
 template <int K>
-__device__ __noinline__ void ppr_close_call(const PprArgs &a, int it, unsigned *s_act) {
-  ppr_close<K>(a, it, s_act);
+__device__ __noinline__ void ppr_close_call(const PprArgs &a, int it, unsigned *s_act,
+                                            double *s_red) {
+  ppr_close<K>(a, it, s_act, s_red);
 }
 
 template <int K>
-__device__ __forceinline__ void close_sweep(const PprArgs &a, int it, unsigned *s_act) {
-  if constexpr (K <= 16) ppr_close_call<K>(a, it, s_act);
-  else ppr_close<K>(a, it, s_act);
+__device__ __forceinline__ void close_sweep(const PprArgs &a, int it, unsigned *s_act,
+                                            double *s_red) {
+  if constexpr (K <= 16) ppr_close_call<K>(a, it, s_act, s_red);
+  else ppr_close<K>(a, it, s_act, s_red);
 }
 
 // All sweeps in one cooperative launch, a bounded grid barrier between them.
-template <int K, typename T>
+// SP: the first kSparseSweeps sweeps of a solve.  x starts as one vertex per vector, so
+// sweep 0 gathers from k vertices and sweep 1 from their out-neighbours.  These sweeps
+// test a bit per source (1 << nz_shift vertices share one, so that the map is at most
+// 128 KB and stays in L1) instead of gathering its row of zeros, skip a round of
+// gathers when no lane has a live source, and leave alone the rows that are 0 and
+// stay 0; the results are the same bits.  A row that becomes non-zero sets its bit,
+// which at worst makes another warp gather its zeros in the same sweep.  From sweep 2
+// on most rows are non-zero; the others follow in a launch of their own (it0 =
+// kSparseSweeps), which ends at once when the solve is over or stopped for packing.
+// Sweep loop, RMAT, dense / sparse start: 2^22 vertices k = 8 (13 sweeps) 6.39 / 5.99
+// ms, 1,000,003 vertices k = 100 (31) 13.2 / 12.5, 300,007 k = 30 (13) 1.37 / 1.17.
+template <int K, typename T, bool SP>
 __global__ void __launch_bounds__(kPprBlock, Shape<K>::min_ctas) k_ppr(PprArgs a) {
   constexpr int L = Shape<K>::L, C = Shape<K>::C;
   extern __shared__ double s_red[];  // [2][warps][K]
@@ -478,9 +578,11 @@ __global__ void __launch_bounds__(kPprBlock, Shape<K>::min_ctas) k_ppr(PprArgs a
   int sd[C];  // seed vertices of this lane's components (-1: padding)
 #pragma unroll
   for (int c = 0; c < C; ++c) sd[c] = a.seed[lq * C + c];
-  int it = 0;
-  while (it < a.max_iter) {
-    ppr_sweep<K, T>(a, it, sd, s_red);
+  int it = SP ? 0 : a.it0;
+  if (!SP && it > 0 && (__ldcg(a.status) != 0 || __ldcg(a.status + 2) != 1)) return;
+  const int end = SP ? min(a.max_iter, kSparseSweeps) : a.max_iter;
+  while (it < end) {
+    ppr_sweep<K, T, SP>(a, it, sd, s_red);
     // Grid barrier; the last CTA closes the sweep.
     if (threadIdx.x == 0) {
       s_gen = ld_acquire(a.bar + 1);
@@ -491,7 +593,7 @@ __global__ void __launch_bounds__(kPprBlock, Shape<K>::min_ctas) k_ppr(PprArgs a
     __syncthreads();
     if (s_state == 1) {
       __threadfence();
-      close_sweep<K>(a, it, s_act);
+      close_sweep<K>(a, it, s_act, s_red);
       if (threadIdx.x == 0) {
         atomicExch(a.bar, 0u);
         __threadfence();
@@ -547,7 +649,7 @@ __global__ void __launch_bounds__(kPprBlock, Shape<K>::min_ctas) k_ppr_step(PprA
   int sd[C];
 #pragma unroll
   for (int c = 0; c < C; ++c) sd[c] = a.seed[lq * C + c];
-  ppr_sweep<K, T>(a, it, sd, s_red);
+  ppr_sweep<K, T, false>(a, it, sd, s_red);
   if (threadIdx.x == 0) {
     __threadfence();
     s_last = atomicAdd(a.bar, 1u) == gridDim.x - 1;
@@ -555,7 +657,7 @@ __global__ void __launch_bounds__(kPprBlock, Shape<K>::min_ctas) k_ppr_step(PprA
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  close_sweep<K>(a, it, s_act);
+  close_sweep<K>(a, it, s_act, s_red);
   if (threadIdx.x == 0) {
     atomicExch(a.bar, 0u);
     a.status[1] = it + 1;
@@ -573,6 +675,7 @@ __global__ void k_ppr_init(PprArgs a) {
     if (v >= 0) {
       const int od = a.outdeg[v];
       a.x[(size_t)v * K + q] = 1.0f;
+      if (a.nz) nz_mark(a, v);
       store_c(reinterpret_cast<T *>(a.c0) + (size_t)v * K + q, od > 0 ? 1.0f / (float)od : 0.f);
       a.dang[q] = od == 0 ? 1.0 : 0.0;
     } else {
@@ -873,6 +976,7 @@ int packets_for(gpr_graph *g, int R, long long want, cudaStream_t st, int **pk, 
 
 struct PprKernels {
   const void *solve;  // persistent: all sweeps in one cooperative launch
+  const void *start;  // persistent: the first two sweeps of a solve
   const void *step;   // one sweep per launch (graph mode)
   void (*init)(PprArgs);
   void (*scatter)(int, int, const int *, const float *, float *);
@@ -881,7 +985,8 @@ struct PprKernels {
 
 template <int K, typename T>
 PprKernels kernels_for() {
-  return {(const void *)k_ppr<K, T>, (const void *)k_ppr_step<K, T>, k_ppr_init<K, T>,
+  return {(const void *)k_ppr<K, T, false>, (const void *)k_ppr<K, T, true>,
+          (const void *)k_ppr_step<K, T>, k_ppr_init<K, T>,
           k_ppr_scatter<K>, k_ppr_refine_init<K>};
 }
 
@@ -982,12 +1087,12 @@ extern "C" int gpr_ppr(gpr_graph *g, int k, const int *h_seeds, float *any_x,
   GPR_TRY(build_chunk_table(g, b_dmax, b_chunk, st));
   const long long units =
       (long long)g->b_nchunks + gpr::ceil_div((long long)L.n_nz - g->b_nlong, R);
-  auto grid_of = [&](const PprKernels &kk, int Kx, long long units_x, int *grid) -> int {
+  auto grid_of = [&](const void *kernel, int Kx, long long units_x, int *grid) -> int {
     const size_t smem_x = sizeof(double) * 2 * (kPprBlock / 32) * Kx;
     int per_sm = 0;
-    GPR_CUDA(cudaFuncSetAttribute(kk.solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    GPR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem_x));
-    GPR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kk.solve, kPprBlock, smem_x));
+    GPR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPprBlock, smem_x));
     if (per_sm < 1) {
       gpr::set_error("gpr_ppr: kernel cannot be resident");
       return GPR_ECUDA;
@@ -997,8 +1102,13 @@ extern "C" int gpr_ppr(gpr_graph *g, int k, const int *h_seeds, float *any_x,
     return GPR_OK;
   };
   int G32 = 0, G16 = 0;
-  GPR_TRY(grid_of(k32, K, units, &G32));
-  if (bf16) GPR_TRY(grid_of(k16, K, units, &G16));
+  GPR_TRY(grid_of(k32.solve, K, units, &G32));
+  if (bf16) GPR_TRY(grid_of(k16.solve, K, units, &G16));
+  // the two first sweeps (persistent form only; at most as many CTAs as the others)
+  int Gs = 0;
+  GPR_TRY(grid_of(bf16 ? k16.start : k32.start, K, units, &Gs));
+  Gs = std::min(Gs, bf16 ? G16 : G32);
+  const bool sparse_start = o.loop != GPR_LOOP_GRAPH && o.max_iter > 0;
   const int Gmax = std::max(G32, G16);
   // About 32 packets per warp of the larger grid: fine enough that the end
   // of a sweep is not held by one warp's last packet (measured on RMAT s22:
@@ -1076,6 +1186,12 @@ extern "C" int gpr_ppr(gpr_graph *g, int k, const int *h_seeds, float *any_x,
   a.damp = o.damping;
   a.max_iter = max_iter;
   a.timeout_ns = (long long)(o.timeout_s * 1e9);
+  if (sparse_start) {
+    while (((long long)m >> a.nz_shift) >= kNzBits) ++a.nz_shift;
+    const size_t words = (size_t)(((long long)m >> a.nz_shift) / 32 + 1);
+    GPR_TRY(B.get(&a.nz, words, "ppr sparse map"));
+    GPR_CUDA(cudaMemsetAsync(a.nz, 0, 4 * words, st));
+  }
   int launches = 0;
   // Graph mode: the sweep loop as one CUDA graph, a while node whose body is
   // one k_ppr_step launch (the kernel clears the condition when the phase is
@@ -1123,7 +1239,8 @@ extern "C" int gpr_ppr(gpr_graph *g, int k, const int *h_seeds, float *any_x,
   // One phase: sweeps until every vector's change is below `tol`, in one
   // cooperative launch, or (GPR_LOOP_GRAPH, or when the grid cannot be
   // co-resident) in the graph loop.  The first phase (`mark`) records the
-  // start event of the sweep loop right before its launch.
+  // start event of the sweep loop right before its launch.  With a.nz set (the first
+  // phase) the sparse kernel runs the first sweeps.
   auto phase = [&](const PprKernels &kk, int G, int Kx, double tol, bool mark, int *sweeps,
                    std::vector<int> *it_out, int *stop) -> int {
     const size_t smem = sizeof(double) * 2 * (kPprBlock / 32) * Kx;
@@ -1135,14 +1252,27 @@ extern "C" int gpr_ppr(gpr_graph *g, int k, const int *h_seeds, float *any_x,
     if (mark && (max_iter <= 0 || !graph_mode)) GPR_CUDA(cudaEventRecord(g->e2, st));
     if (max_iter > 0 && !graph_mode) {
       void *args[] = {&a};
-      cudaError_t e = cudaLaunchCooperativeKernel(kk.solve, dim3(G), dim3(kPprBlock), args, smem, st);
+      cudaError_t e = cudaSuccess;
+      a.it0 = 0;
+      if (a.nz) {
+        a.bar_expect += Gs - G;
+        e = cudaLaunchCooperativeKernel(kk.start, dim3(Gs), dim3(kPprBlock), args, smem, st);
+        a.bar_expect += G - Gs;
+        a.nz = nullptr;
+        if (e == cudaSuccess) {
+          ++launches;
+          a.it0 = std::min(a.max_iter, kSparseSweeps);
+        }
+      }
+      const bool rest = e == cudaSuccess && a.it0 < a.max_iter;
+      if (rest) e = cudaLaunchCooperativeKernel(kk.solve, dim3(G), dim3(kPprBlock), args, smem, st);
       if (e == cudaErrorCooperativeLaunchTooLarge) {
         cudaGetLastError();
         graph_mode = true;
       } else if (e != cudaSuccess) {
         gpr::set_error("gpr_ppr: %s", cudaGetErrorString(e));
         return GPR_ECUDA;
-      } else {
+      } else if (rest) {
         ++launches;
       }
     }
@@ -1194,7 +1324,7 @@ extern "C" int gpr_ppr(gpr_graph *g, int k, const int *h_seeds, float *any_x,
       last_K = Kc;
       for (int q = 0; q < Kc; ++q)
         if (slot_of[q] >= 0) (*it_total)[slot_of[q]] += itc[q];
-      const bool packed = Kc != K;
+      const bool packed = xc != x;
       if (stop != 2 || *sweeps >= max_iter) {
         if (packed) {  // the packed layout's results back into the master
           k_ppr_unpack<<<(unsigned)gpr::ceil_div((long long)m * Kc, 256), 256, 0, st>>>(
@@ -1246,7 +1376,7 @@ extern "C" int gpr_ppr(gpr_graph *g, int k, const int *h_seeds, float *any_x,
       const int Rn = 32 / (Kc / 4);
       const long long units_n =
           (long long)g->b_nchunks + gpr::ceil_div((long long)L.n_nz - g->b_nlong, Rn);
-      GPR_TRY(grid_of(kc, Kc, units_n, &Gc));
+      GPR_TRY(grid_of(kc.solve, Kc, units_n, &Gc));
       int *pk = nullptr, npk = 0;
       GPR_TRY(packets_for(g, Rn, (long long)Gc * (kPprBlock / 32) * 32, st, &pk, &npk));
       a.pk = pk;

@@ -206,3 +206,52 @@ def test_ppr_packing_with_a_sweep_cap(G, O):
     assert sta.iterations == stb.iterations == 9
     np.testing.assert_array_equal(ita, itb)
     assert np.abs(xa - xb).max() <= 1e-6
+
+
+@pytest.mark.parametrize("k", [1, 2, 5, 8, 9, 40, 100])
+def test_ppr_sparse_sweeps(G, O, k):
+    """The first two sweeps skip sources and rows that are 0.  Seeds in the giant
+    component, in small closed sets of vertices (a pair pointing at each other, a
+    triangle with a dangling tail) and without out-edges: the bits of the graph loop,
+    whose sweeps are all dense, and the oracle's bars."""
+    from graphs import in_csr
+    rng = np.random.default_rng(k)
+    rp0, col0, od0 = O.rmat_graph(12, 8, seed=41)
+    n = len(rp0) - 1
+    dst = np.repeat(np.arange(n), np.diff(rp0))
+    pairs = 30
+    a = n + 2 * np.arange(pairs)
+    t = n + 2 * pairs
+    src = np.concatenate([col0, a, a + 1, [t, t + 1, t + 2, t + 2]])
+    dst = np.concatenate([dst, a + 1, a, [t + 1, t + 2, t, t + 3]])
+    m = t + 4
+    rp, col, od = in_csr(m, src, dst)
+    odd = np.concatenate([a, [t, t + 2, t + 3]])
+    some = np.flatnonzero((np.diff(rp) > 0) & (od > 0))
+    seeds = np.where(np.arange(k) % 3 == 0, rng.choice(odd, k), rng.choice(some, k)).astype(np.int32)
+    ref, ref_it = O.ppr_f64(rp, col, od, seeds, tol=1e-6, max_iter=100)
+    assert ref_it.max() > 50
+    with G.Graph(rp, col, od, batched=True) as g:
+        x, it, st = g.ppr(seeds, tol=1e-6, max_iter=100)
+        y, it_y, _ = g.ppr(seeds, tol=1e-6, max_iter=100, loop=G.LOOP_GRAPH)
+        z, it_z, _ = g.ppr(seeds, tol=0.0, max_iter=20, ppr_repack=False)
+        w, it_w, _ = g.ppr(seeds, tol=0.0, max_iter=20, loop=G.LOOP_GRAPH, ppr_repack=False)
+        b, it_b, _ = g.ppr(seeds, tol=1e-6, max_iter=200, precision=G.PREC_BF16)
+    assert np.array_equal(x, y) and np.array_equal(it, it_y)
+    assert np.array_equal(z, w) and np.array_equal(it_z, it_w)
+    assert np.all(l1_per_vector(x, ref) <= 1e-5)
+    assert np.all(np.abs(it - ref_it) <= 1)
+    fixed, _ = O.ppr_f64(rp, col, od, seeds, tol=1e-12, max_iter=400)
+    assert np.all(l1_per_vector(b, fixed) <= 1e-5)
+
+
+@pytest.mark.parametrize("max_iter", [1, 2, 3, 17])
+def test_ppr_sweep_limits_around_the_sparse_start(G, O, max_iter):
+    """A limit inside, at the end of and just behind the two sparse sweeps."""
+    rp, col, od = O.rmat_graph(11, 8, seed=43)
+    seeds = O.uniform_int(6, 5, len(rp) - 1)
+    with G.Graph(rp, col, od, batched=True) as g:
+        x, it, st = g.ppr(seeds, tol=0.0, max_iter=max_iter)
+        y, it_y, _ = g.ppr(seeds, tol=0.0, max_iter=max_iter, loop=G.LOOP_GRAPH)
+    assert st.iterations == max_iter and np.all(it == max_iter)
+    assert np.array_equal(x, y) and np.array_equal(it, it_y)
