@@ -724,6 +724,18 @@ __global__ void k_ppr_scatter(int m, int k, const int *__restrict__ perm,
   out[(size_t)perm[v] * k + q] = x[(size_t)v * K + q];
 }
 
+// The same for k a multiple of 4 and a 16-byte aligned `out`: 16 bytes per thread.
+// What follows the sweep loop, 1,000,003 x 100: 376 -> 185 us, 2^22 x 8: 144 -> 89 us.
+template <int K>
+__global__ void k_ppr_scatter4(int m, int k4, const int *__restrict__ perm,
+                               const float4 *__restrict__ x, float4 *out) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= (long long)m * k4) return;
+  const long long v = t >> 32 ? t / k4 : (long long)((unsigned)t / (unsigned)k4);
+  const int q = (int)(t - v * k4);
+  out[(size_t)perm[v] * k4 + q] = x[(size_t)v * (K / 4) + q];
+}
+
 // Packing of the still-updating vectors into a narrower layout of Kn slots:
 // slot j of the new layout takes slot sel[j] of the old one (x, the
 // contributions the next sweep reads, including the zero sentinel row m, the
@@ -980,6 +992,7 @@ struct PprKernels {
   const void *step;   // one sweep per launch (graph mode)
   void (*init)(PprArgs);
   void (*scatter)(int, int, const int *, const float *, float *);
+  void (*scatter4)(int, int, const int *, const float4 *, float4 *);
   void (*refine_init)(PprArgs, const double *);
 };
 
@@ -987,7 +1000,7 @@ template <int K, typename T>
 PprKernels kernels_for() {
   return {(const void *)k_ppr<K, T, false>, (const void *)k_ppr<K, T, true>,
           (const void *)k_ppr_step<K, T>, k_ppr_init<K, T>,
-          k_ppr_scatter<K>, k_ppr_refine_init<K>};
+          k_ppr_scatter<K>, k_ppr_scatter4<K>, k_ppr_refine_init<K>};
 }
 
 int pick_k(int k) {
@@ -1426,8 +1439,12 @@ extern "C" int gpr_ppr(gpr_graph *g, int k, const int *h_seeds, float *any_x,
     GPR_TRY(B.get(&xout, (size_t)m * k, "ppr output staging"));
     dout = xout;
   }
-  k32.scatter<<<(unsigned)gpr::ceil_div((long long)m * k, 256), 256, 0, st>>>(m, k, L.perm, x,
-                                                                              dout);
+  if (k % 4 == 0 && reinterpret_cast<uintptr_t>(dout) % 16 == 0)
+    k32.scatter4<<<(unsigned)gpr::ceil_div((long long)m * (k / 4), 256), 256, 0, st>>>(
+        m, k / 4, L.perm, reinterpret_cast<const float4 *>(x), reinterpret_cast<float4 *>(dout));
+  else
+    k32.scatter<<<(unsigned)gpr::ceil_div((long long)m * k, 256), 256, 0, st>>>(m, k, L.perm, x,
+                                                                                dout);
   ++launches;
   GPR_CUDA(cudaGetLastError());
   GPR_CUDA(cudaEventRecord(g->e1, st));

@@ -255,3 +255,23 @@ def test_ppr_sweep_limits_around_the_sparse_start(G, O, max_iter):
         y, it_y, _ = g.ppr(seeds, tol=0.0, max_iter=max_iter, loop=G.LOOP_GRAPH)
     assert st.iterations == max_iter and np.all(it == max_iter)
     assert np.array_equal(x, y) and np.array_equal(it, it_y)
+
+
+@pytest.mark.parametrize("k,offset", [(4, 0), (4, 1), (6, 0), (100, 0), (100, 3), (128, 0)])
+def test_ppr_output_layouts(G, O, k, offset):
+    """x goes back 16 bytes at a time when k is a multiple of 4 and the caller's buffer
+    starts on 16 bytes, else one by one: the same values, nothing written outside."""
+    torch = pytest.importorskip("torch")
+    rp, col, od = O.rmat_graph(9, 8, seed=44)
+    m = len(rp) - 1
+    seeds = O.uniform_int(k, 6, m)
+    with G.Graph(rp, col, od, batched=True) as g:
+        ref, _, _ = g.ppr(seeds, tol=0.0, max_iter=4)
+        buf = torch.full((m * k + 8,), -7.0, device="cuda")
+        out = buf[offset:offset + m * k]
+        torch.cuda.synchronize()
+        g.ppr(seeds, out=out, tol=0.0, max_iter=4)
+        torch.cuda.synchronize()
+    got = buf.cpu().numpy()
+    assert np.array_equal(got[offset:offset + m * k].reshape(m, k), ref)
+    assert np.all(got[:offset] == -7.0) and np.all(got[offset + m * k:] == -7.0)
