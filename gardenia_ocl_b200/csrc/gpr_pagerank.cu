@@ -611,7 +611,15 @@ struct SweepKernels {
 };
 using bf16 = __nv_bfloat16;
 // Indices 0..7: the FP32 variants a caller selects with opts.variant;
-// index kBf16Kernel: the BF16-contribution kernel of the mixed form.
+// index kBf16Kernel: the BF16-contribution kernel of the mixed form; index
+// kLargeKernel: variant 0's for graphs of kLargeEdges edges and more.  There eight
+// entries of a slice in flight per lane are faster than sixteen (half-empty batches of
+// short rows cost issue slots, and other warps hide the latency), below slower; the
+// order of additions is the same.  Sweep loops, RMAT, 16 / 8 entries: 400,009 vertices
+// (5.6M edges) 787 / 813 us, 700,001 (4.7M) 864 / 848, 1,000,003 (15M) 1758 / 1667,
+// 1,500,007 (13M) 1703 / 1614, 3,000,017 (41M) 4848 / 4649, 2^24 (263M, 8 sweeps) 6184 /
+// 6045; 6 or 4 entries gained nothing more, and the next batch's indices loaded
+// before the current one's gathers lost 2 to 5% against 8.
 const SweepKernels kKernels[] = {
     {(const void *)k_pr_hot<16, 4, true, 1, float>, k_pr_step<16, 4, float>, 1, 227328, 4},
     {(const void *)k_pr_hot<8, 2, false, 1, float>, k_pr_step<8, 2, float>, 1, 227328, 4},
@@ -622,6 +630,7 @@ const SweepKernels kKernels[] = {
     {(const void *)k_pr_hot<8, 2, false, 2, float>, k_pr_step<8, 2, float>, 2, 98304, 4},
     {(const void *)k_pr_hot<8, 2, true, 2, float>, k_pr_step<8, 2, float>, 2, 98304, 4},
     {(const void *)k_pr_hot<16, 4, true, 1, bf16>, k_pr_step<16, 4, bf16>, 1, 227328, 2},
+    {(const void *)k_pr_hot<8, 4, true, 1, float>, k_pr_step<16, 4, float>, 1, 227328, 4},
 };
 constexpr int kHotBlock = 1024;
 // A small graph takes a CTA for every 8 units, up to one per SM: a sweep is then
@@ -630,11 +639,18 @@ constexpr int kHotBlock = 1024;
 constexpr int kUnitsPerCta = 8;
 constexpr int kNumVariants = 8;
 constexpr int kBf16Kernel = 8;
+constexpr int kLargeKernel = 9;
+constexpr long long kLargeEdges = 1LL << 23;
 constexpr int kNumKernels = sizeof(kKernels) / sizeof(kKernels[0]);
 // The BF16 phase of the mixed form stops once the L1 change is below this
 // (or the caller's tol if larger): about where BF16 rounding of the
 // contributions stops the residual from falling further.
 constexpr double kBf16Tol = 1e-3;
+
+// The FP32 sweep kernel for a caller's variant.
+int sweep_kernel(const gpr_graph *g, int variant) {
+  return variant == 0 && g->L.nnz >= kLargeEdges ? kLargeKernel : variant;
+}
 
 // Contributions kernel ki stages in shared memory: the caller's hot budget in
 // bytes, covering the sentinel slot m when the whole array fits, a multiple
@@ -1191,11 +1207,11 @@ int pagerank_impl(gpr_graph *g, float *any_scores, const gpr_pr_opts *opts_in,
                        "co-resident grid");
         rc = GPR_EINVAL;
       } else {
-        rc = solve_impl(g, d_scores, o, o.variant, &st_local);
+        rc = solve_impl(g, d_scores, o, sweep_kernel(g, o.variant), &st_local);
       }
     }
   } else if (o.precision == GPR_PREC_FP32) {
-    rc = solve_impl(g, d_scores, o, o.variant, &st_local);
+    rc = solve_impl(g, d_scores, o, sweep_kernel(g, o.variant), &st_local);
   } else {
     // Mixed form: BF16 contributions (twice the entries in the shared-memory
     // cache, half the bytes per gather) until the change is below
@@ -1207,7 +1223,7 @@ int pagerank_impl(gpr_graph *g, float *any_scores, const gpr_pr_opts *opts_in,
     if (rc == GPR_OK) {
       gpr_pr_opts o2 = o;
       o2.max_iter = std::max(0, o.max_iter - s1.iterations);
-      rc = solve_impl(g, d_scores, o2, o.variant, &s2);
+      rc = solve_impl(g, d_scores, o2, sweep_kernel(g, o.variant), &s2);
       st_local = s2;
       st_local.iterations = s1.iterations + s2.iterations;
       st_local.refine_iterations = s2.iterations;

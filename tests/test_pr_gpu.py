@@ -320,3 +320,18 @@ def test_default_bins_by_size(G, O, deg):
         b, _, _, _ = mg.pagerank(tol=0.0, max_iter=6)
     small, _, _, _ = solve(G, rp2, col2, od2, tol=0.0, max_iter=6)
     assert np.array_equal(b[:m], s) and np.array_equal(b[m:], small)
+
+
+def test_large_graph_kernel_has_the_same_bits(G, O):
+    # From 2^23 edges up variant 0 keeps eight entries of a slice in flight instead of
+    # sixteen; the order of additions is that of the other variants with 16-byte
+    # chunk loads of the same count (variant 4), so the scores are the same bits.
+    torch = pytest.importorskip("torch")
+    csr = G.gen_rmat(20, 10, seed=8)
+    assert csr.nnz >= 1 << 23
+    with G.Graph(csr.rowptr, csr.col, csr.third, m=csr.m, nnz=csr.nnz) as g:
+        a, st_a = g.pagerank(tol=0.0, max_iter=4)
+        b, st_b = g.pagerank(tol=0.0, max_iter=4, variant=4)
+        c, _ = g.pagerank(tol=0.0, max_iter=4, loop=G.LOOP_GRAPH)
+    assert np.array_equal(a, b) and np.array_equal(a, c)
+    csr.close()
