@@ -22,7 +22,7 @@ void set_error(const char *fmt, ...) {
 }
 
 // Block cache of device allocations.  One-shot solver calls (the reference's
-// PRSolver shape: copy in, build, solve, free) make some sixty allocations each, of
+// PRSolver shape: copy in, build, solve, free) make dozens of allocations each, of
 // a few bytes to gigabytes: mapping and unmapping the large ones makes cudaMalloc
 // / cudaFree slow and erratic, and every cudaFree of a small one waits for the
 // device.  Blocks are kept after dfree and handed out again: large ones (kCacheMin

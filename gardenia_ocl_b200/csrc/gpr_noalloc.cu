@@ -93,8 +93,7 @@ __global__ void k_na_prologue(NoAllocArgs a) {
 }
 
 // acc + v[lo] + ... + v[hi - 1] in order.  The loads of a batch are issued before
-// its additions, so a value costs an addition's latency and not a load's as well
-// (about 6 cycles against 33).
+// its additions, so a value costs an addition's latency and not a load's as well.
 __device__ __forceinline__ float add_in_order(const float *v, int lo, int hi, float acc) {
   for (; lo < hi; lo += 16) {
     float x[16];
@@ -111,8 +110,8 @@ __device__ __forceinline__ float add_in_order(const float *v, int lo, int hi, fl
 // lanes' strides fall on different shared-memory banks.
 constexpr int kOrdV = 31;
 // Rows with more values than this in a staged tile are added by their warp.
-// One thread adds at about 6 cycles a value; the warp's step costs 450 cycles
-// for up to 992 values, and a row starts with one or two sequential stretches.
+// A shorter row gains nothing from a warp: its first steps, with a new binade after
+// every doubling of the sum, mostly add one by one.
 constexpr int kOrdMin = 384;
 
 // acc + v[lo] + v[lo + 1] + ... + v[hi - 1], each addition rounded to nearest
