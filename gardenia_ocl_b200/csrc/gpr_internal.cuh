@@ -325,12 +325,14 @@ struct gpr_graph {
   int blocked_carve = 0;       // shared-memory share of the SM for them, percent
   int *tq = nullptr;
   unsigned *fx_max = nullptr;
+  double *fx_part = nullptr;   // per-CTA sums of |score| (k_sum_abs)
   alignas(8) unsigned char loop_args[512] = {0};
 };
 
 namespace gpr {
 // The push solver's solve in the blocked form (gpr_pagerank.cu).  kPushFallback: the
-// form does not apply (a non-finite score, no co-resident grid); nothing was done.
+// form does not apply (a non-finite score, too much mass for its precision, no
+// co-resident grid); nothing was done.
 constexpr int kPushFallback = 101;
 int push_blocked(gpr_graph *g, float *any_scores, const gpr_pr_opts &opts, gpr_pr_stats *stats);
 

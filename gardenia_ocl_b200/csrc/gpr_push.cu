@@ -16,10 +16,11 @@
 // memory.  RMAT, 3,000,017 vertices, edge factor 16, tol 1e-6: 12.7 ms per solve with
 // one L2 reduction per edge outside the hot prefix, 4.9 ms this way; sweep loops of
 // 2,000 / 20,000 / 100,000 / 300,000 / 1,000,003 vertices 449 / 635 / 1540 / 1999 /
-// 3888 us before and 233 / 360 / 932 / 1242 / 2089 us after, so it is used at all sizes.
+// 3888 us before and 233 / 360 / 932 / 1242 / 2089 us after, so it is used at all sizes,
+// from every start whose mass its fixed point holds to better than FP32 (solve_impl).
 //
-// Where that form does not apply (a non-finite score, no scratch for its layout) the
-// edges go one by one: the in-CSR's edges as a list sorted by source (relabelled ids,
+// Where that form does not apply (a non-finite score, too much mass, damping 1, no
+// scratch for its layout) the edges go one by one: the in-CSR's edges as a list sorted by source (relabelled ids,
 // built on first use), so each warp reads 32 consecutive edges -- equal work
 // for every warp, and the contribution loads of one warp fall on a few
 // neighbouring sources.  One persistent cooperative launch for all sweeps:

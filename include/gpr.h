@@ -84,13 +84,20 @@ typedef struct {
  *   BLOCKED  rows (all but the hubs, gpr_layout_opts.blocked_long) are summed
  *            block by block from source-ordered edges (far fewer memory
  *            requests on large graphs), in 64-bit fixed point: the exact sum
- *            of the FP32 contributions rounded once to 2^-S (S >= 31, chosen
- *            per solve from the edge count and the largest score), then to
- *            FP32.  Deterministic.  Needs a graph created with
- *            GPR_LAYOUT_BLOCKED and the persistent loop.
+ *            of the FP32 contributions rounded once to 2^-S (chosen per
+ *            solve from the edge count and m x the largest initial score: about
+ *            28 + log2(edges) for scores of 1/m, fewer the further m x that score
+ *            is above 1, 31 or more up to m x score = 2^31), then to FP32.  With a
+ *            small S (all scores 1, one vertex that holds all of the mass) scores
+ *            of about 1/m keep few correct digits.  Deterministic.  Needs a graph
+ *            created with GPR_LAYOUT_BLOCKED and the persistent loop.
  *   AUTO     BLOCKED when the graph has its layout, at least 50,331,648 edges
  *            (below that EXACT measured faster: RMAT scale 21 3.6 vs 3.9 ms,
- *            scale 22 7.6 vs 6.8 ms) and the persistent loop runs, else EXACT. */
+ *            scale 22 7.6 vs 6.8 ms) and the persistent loop runs, else EXACT.
+ *            Where the S above would show in the scores, BLOCKED takes one from
+ *            the sum of the initial |scores| that does not (1/m, one vertex, an
+ *            earlier solution: any start of mass about 1); where there is none
+ *            (all ones on a large graph, damping 1), EXACT solves. */
 typedef enum {
   GPR_FORM_AUTO = 0,
   GPR_FORM_EXACT = 1,
@@ -219,12 +226,15 @@ int gpr_ppr(gpr_graph *g, int k, const int *h_seeds, float *any_x,
  * scatter each source's contribution to its out-neighbours with atomic adds.
  * Same recurrence and stop rule as gpr_pagerank (so the two directions solve
  * the same problem).  The first call builds the blocked layout (edges in source
- * order, cut by destination block; see gpr_form) and every solve adds the
+ * order, cut by destination block; see gpr_form) and a solve adds the
  * contributions to their destinations' accumulators in shared memory, in 64-bit
- * fixed point: deterministic.  With a non-finite initial score, or without the
- * scratch for that layout, edges sorted by source add one by one in FP32, and the
- * last bits of the result vary from run to run.  The graph must be created with
- * GPR_LAYOUT_PUSH (or GPR_LAYOUT_BATCHED); FP32 only. */
+ * fixed point whose rounding is below that of the FP32 scores: deterministic.
+ * Where fixed point cannot hold them so (a non-finite initial score, more mass
+ * than its 62 bits leave room for -- all ones on a large graph --, damping 1), or
+ * without the scratch for that layout, edges sorted by source add one by one in
+ * FP32, and the last bits of the result vary from run to run.  opts->form and
+ * opts->variant are not read.  The graph must be created with GPR_LAYOUT_PUSH
+ * (or GPR_LAYOUT_BATCHED); FP32 only. */
 int gpr_pagerank_push(gpr_graph *g, float *any_scores, const gpr_pr_opts *opts,
                       gpr_pr_stats *stats);
 

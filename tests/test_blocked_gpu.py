@@ -266,3 +266,28 @@ def test_graph_zoo_is_the_fixed_point_recurrence(G, O, kind, seed):
     assert abs(st.iterations - ref_it) <= 1
     s64, _, _ = O.pr_f64(rp, col, od, tol=0.0, max_iter=st.iterations)
     assert np.all(np.abs(s - ref) <= ABS_TOL + np.abs(ref - s64))
+
+
+@pytest.mark.parametrize("kind", ["one_vertex", "ones", "solution"])
+def test_auto_keeps_fp32_precision_from_any_start(G, O, kind):
+    """From 50,331,648 edges on AUTO solves in blocks; from a start whose largest score is
+    far above 1/m it takes the exponent from the mass, or the exact order.  Per vertex
+    within (8 + 4 sqrt(k)) 2^-24 of the FP64 recurrence (a few roundings of the score,
+    contributions and update; k terms in FP32 in any order another sqrt(k) or so)."""
+    csr = G.gen_rmat(22, 14, seed=3)
+    rp, col, od = csr.rowptr.to_numpy(), csr.col.to_numpy(), csr.third.to_numpy()
+    m = csr.m
+    assert csr.nnz >= 50331648
+    s0 = np.ones(m, dtype=np.float32)
+    if kind == "one_vertex":
+        s0[:] = 0.0
+        s0[int(np.argmax(od))] = 1.0
+    with G.Graph(csr.rowptr, csr.col, csr.third, m=m, nnz=csr.nnz, blocked=True) as g:
+        if kind == "solution":
+            s0, _ = g.pagerank(tol=1e-6, max_iter=100)
+        s, st = g.pagerank(s0.copy(), tol=0.0, max_iter=8)
+    csr.close()
+    assert st.iterations == 8
+    ref, _, _ = O.pr_f64(rp, col, od, tol=0.0, max_iter=8, init=s0)
+    bound = (8 + 4 * np.sqrt(np.diff(rp))) * 2.0 ** -24
+    assert np.all(np.abs(s - ref) <= bound * ref)

@@ -104,3 +104,42 @@ def test_push_non_finite_scores(G, O):
     assert st.iterations == 2 and not fin.all()
     assert np.array_equal(fin, np.isfinite(s))
     assert np.abs(s[fin] - ref[fin]).max() <= 1e-6
+
+
+def far_start(kind, m, rp, col, od, O):
+    """Finite starts whose largest score is far above 1/m."""
+    rng = np.random.default_rng(len(kind))
+    if kind == "one_vertex":
+        s = np.zeros(m, dtype=np.float32)
+        s[int(np.argmax(od))] = 1.0
+    elif kind == "ones":
+        s = np.ones(m, dtype=np.float32)
+    elif kind == "random":
+        s = rng.random(m).astype(np.float32)
+    elif kind == "solution":
+        s = O.pr_f64(rp, col, od, tol=1e-9, max_iter=200)[0].astype(np.float32)
+    else:  # scores over some thirty binades, total 1
+        w = np.exp(rng.normal(0, 6, m))
+        s = (w / w.sum()).astype(np.float32)
+    return s
+
+
+@pytest.mark.parametrize("kind", ["one_vertex", "ones", "random", "solution", "wide"])
+def test_push_from_starts_far_from_uniform(G, O, kind):
+    """The precision of FP32 contributions whatever the finite start.  A score is at
+    least the base (1-d)/m; its contributions, update and 20 sweeps of sources'
+    errors are a few roundings of 2^-24, and k terms added in any order in FP32
+    another sqrt(k) or so of them: (8 + 4 sqrt(k)) 2^-24 relative per vertex."""
+    rp, col, od = O.rmat_graph(17, 16, seed=6)
+    m = len(rp) - 1
+    s0 = far_start(kind, m, rp, col, od, O)
+    with G.Graph(rp, col, od, push=True) as g:
+        s, st = g.pagerank_push(s0.copy(), tol=0.0, max_iter=20)
+        t, st_t = g.pagerank_push(s0.copy(), tol=1e-5, max_iter=200)
+    ref, _, _ = O.pr_f64(rp, col, od, tol=0.0, max_iter=20, init=s0)
+    bound = (8 + 4 * np.sqrt(np.diff(rp))) * 2.0 ** -24
+    rel = np.abs(s - ref) / ref
+    assert st.iterations == 20
+    assert np.all(rel <= bound), (rel.max(), np.sort(rel / bound)[-3:])
+    _, n, _ = O.pr_f64(rp, col, od, tol=1e-5, max_iter=200, init=s0)
+    assert abs(st_t.iterations - n) <= 1
