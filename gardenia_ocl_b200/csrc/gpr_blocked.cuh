@@ -8,11 +8,23 @@
 #pragma once
 
 #include "gpr_device.cuh"
+#include "gpr_internal.cuh"
 
 namespace gpr {
 namespace blk {
 
 using namespace gpr::dev;
+
+// |s| summed per CTA: a grid of kSumBlocks CTAs always, so that the sum of `part` is the
+// same on every run.
+static __global__ void __launch_bounds__(256) k_sum_abs(int m, const float *__restrict__ s,
+                                                        double *part) {
+  double t = 0.0;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < m; i += kSumBlocks * 256LL)
+    t += (double)fabsf(s[i]);
+  t = block_sum_double(t);
+  if (threadIdx.x == 0) part[blockIdx.x] = t;
+}
 
 // The blocked rows are summed block by block (gpr_blocked.cu): the CTA that
 // takes a tile zeroes one accumulator per row of the tile's block in shared

@@ -2,9 +2,11 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 #include <stdio.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "gpr.h"
@@ -151,6 +153,30 @@ struct BlockedLayout {
   int *bcnt = nullptr;                   // [n_blocks] tiles done in the current sweep
   long long device_bytes = 0;
 };
+
+// Fixed-point exponent S of the blocked form for a solve whose sweeps hold a total
+// |score| of at most b0 (a sweep maps total mass M to at most (1-d) + d*M, so the
+// larger of 1 and the initial mass bounds them all): a row's sum is at most that, so
+// |sum| * 2^S < 2^63 needs S <= 62 - log2(b0), blocked_cap.  Within that, S puts a
+// typical contribution (about b0 / nnz) near 2^28, so most fit the low 32-bit word of
+// the accumulator; S >= 31 unless b0 > 2^31.
+inline int blocked_cap(double b0) { return 62 - (int)ceil(log2(b0)); }
+
+inline int blocked_shift(long long nnz, double b0) {
+  const int pref = (int)floor(log2(std::max(1.0, (double)nnz) / b0)) + 28;
+  return std::min(blocked_cap(b0), std::max(31, pref));
+}
+
+// The S from which on the rounding to 2^-S is lost in a score's own FP32 rounding:
+// the roundings of a row of k contributions add up to about sqrt(k / 12) * 2^-S, and
+// no score of a sweep from scores >= 0 is below the base (1-d) / m.  With the mean
+// in-degree for k, that error is a quarter of 2^-24 of the base; rows of more
+// in-edges hold more than the base.  No S is enough for d = 1.
+inline double blocked_bits(int m, long long nnz, double d) {
+  return 24.0 + log2((double)m / (1.0 - d)) + 0.5 * log2(std::max(1.0, (double)nnz / m));
+}
+
+constexpr int kSumBlocks = 256;  // CTAs of k_sum_abs
 
 // Rows of the blocked form that stay chunked: the first *row0 rows of the
 // exact-order layout's chunked rows [0, L.n_long), either those with more than

@@ -725,6 +725,8 @@ struct gpr_multigraph {
   gpr::BlockedLayout B;
   bool has_blocked = false, blocked_ok = false;
   int grid_blocked = 0, blocked_ctas = 1, max_gm = 0;
+  double fx_bits = 0.0;   // largest blocked_bits of the graphs at damping 0
+  double *fx_part = nullptr;  // per-CTA sums of |score| (k_sum_abs)
   int blocked_carve = 0;  // shared-memory share of the SM for the blocked kernel, percent
   int *tq = nullptr, *tb = nullptr, *lazy_b = nullptr;
   std::vector<int> lazy_bh;     // graphs with vertices but no tiles
@@ -748,7 +750,8 @@ const void *multi_blocked_kernel(int ctas) {
                    : (const void *)k_multi_blocked<4, 1024, 1>;
 }
 
-// solve_phase status: the blocked form cannot represent these scores
+// solve_phase status: the blocked form cannot represent these scores (as
+// kBlockedFallback of gpr_pagerank.cu)
 constexpr int kMultiBlockedFallback = 100;
 
 void destroy_multi(gpr_multigraph *g) {
@@ -757,7 +760,8 @@ void destroy_multi(gpr_multigraph *g) {
                   g->hb,    g->zb,     g->cap,     g->stop,    g->gdone,  g->lazy,
                   g->gres,  g->s,      g->c0,      g->c1,      g->h0,     g->h1,
                   g->partial, g->cnt,  g->uerr,    g->n_next,  g->bar,    g->status,
-                  g->wq,    g->scores_tmp, g->pk, g->tq, g->tb, g->lazy_b, g->terr, g->fx_max};
+                  g->wq,    g->scores_tmp, g->pk, g->tq, g->tb, g->lazy_b, g->terr, g->fx_max,
+                  g->fx_part};
   for (void *p : ptrs) gpr::dfree(p);
   gpr::free_blocked_layout(&g->B);
   if (g->e0) cudaEventDestroy(g->e0);
@@ -1039,7 +1043,12 @@ int build_multi(gpr_multigraph *g, const int *h_voff, const int *d_rowptr, const
   }
   g->grid = (int)std::max<long long>(1, std::min<long long>(sms, gpr::ceil_div(U, 32)));
   GPR_CUDA(cudaStreamSynchronize(st));
-  for (int r = 0; r < G; ++r) g->max_gm = std::max(g->max_gm, gm[r]);
+  for (int r = 0; r < G; ++r) {
+    g->max_gm = std::max(g->max_gm, gm[r]);
+    const int ug = g->order[r];
+    if (gm[r] > 0)
+      g->fx_bits = std::max(g->fx_bits, gpr::blocked_bits(gm[r], eoff[ug + 1] - eoff[ug], 0.0));
+  }
   if (blo) {
     // Blocked form: the rows with in-edges of each graph (the first rows of
     // its range) in blocks of R rows, never spanning two graphs.
@@ -1068,6 +1077,7 @@ int build_multi(gpr_multigraph *g, const int *h_voff, const int *d_rowptr, const
     GPR_TRY(gpr::dalloc(&g->lazy_b, std::max<size_t>(g->lazy_bh.size(), 1), "graphs without tiles"));
     GPR_TRY(gpr::dalloc(&g->tq, 2, "tile queue"));
     GPR_TRY(gpr::dalloc(&g->fx_max, 1, "largest score"));
+    GPR_TRY(gpr::dalloc(&g->fx_part, gpr::kSumBlocks, "score sums"));
     GPR_CUDA(cudaMemcpyAsync(g->tb, B.range_tiles.data(), sizeof(int) * ((size_t)G + 1),
                              cudaMemcpyHostToDevice, st));
     if (!g->lazy_bh.empty())
@@ -1164,6 +1174,7 @@ int solve_phase(gpr_multigraph *g, float *d_scores, const gpr_pr_opts &o, bool b
   a.n_pk = g->n_pk;
   a.timeout_ns = (long long)(o.timeout_s * 1e9);
   a.cond = 0;
+  int sum_launches = 0;
   if (blocked) {
     const gpr::BlockedLayout &B = g->B;
     GPR_CUDA(cudaMemsetAsync(g->tq, 0, 2 * sizeof(int), st));
@@ -1183,10 +1194,28 @@ int solve_phase(gpr_multigraph *g, float *d_scores, const gpr_pr_opts &o, bool b
     float mx;
     memcpy(&mx, &bits, sizeof(mx));
     if (!isfinite(mx)) return kMultiBlockedFallback;
-    const double b0 = std::max(1.0, (double)g->max_gm * (double)mx);
-    const int cap = 62 - (int)ceil(log2(b0));
-    const int pref = (int)floor(log2(std::max(1.0, (double)g->nnz) / b0)) + 28;
-    const int S = std::min(cap, std::max(31, pref));
+    int S = gpr::blocked_shift(g->nnz, std::max(1.0, (double)g->max_gm * (double)mx));
+    // Where that leaves fewer bits than the largest graph's scores need (a graph whose
+    // mass is on few vertices, an earlier solution with its hubs), the batch's whole
+    // mass bounds each graph's; without room for the bits the form does not apply.
+    // One exponent for graphs of all sizes costs up to 3 bits from 1/m_g as well (512
+    // graphs of 1,000 to 500,000 vertices: S = 45 against 47.7); those are not searched
+    // for.  A caller who asked for the blocked form by name gets the S of the bound.
+    const double bits_needed = g->fx_bits - log2(1.0 - (double)o.damping);
+    if (o.form != GPR_FORM_BLOCKED && (double)S < bits_needed - 3.0) {
+      std::vector<double> part(gpr::kSumBlocks);
+      gpr::blk::k_sum_abs<<<gpr::kSumBlocks, 256, 0, st>>>(M, d_scores, g->fx_part);
+      GPR_CUDA(cudaGetLastError());
+      GPR_CUDA(cudaMemcpyAsync(part.data(), g->fx_part, sizeof(double) * gpr::kSumBlocks,
+                               cudaMemcpyDeviceToHost, st));
+      GPR_CUDA(cudaStreamSynchronize(st));
+      double mass = 0.0;
+      for (double x : part) mass += x;
+      if (bits_needed > (double)gpr::blocked_cap(std::max(1.0, mass * (1.0 + 1e-9))))
+        return kMultiBlockedFallback;
+      S = (int)ceil(bits_needed);
+      ++sum_launches;
+    }
     a.fx_scale = ldexpf(1.f, S);
     a.fx_inv = ldexp(1.0, -S);
     a.tb = g->tb;
@@ -1309,7 +1338,7 @@ int solve_phase(gpr_multigraph *g, float *d_scores, const gpr_pr_opts &o, bool b
   out->iterations = max_cap > 0 ? hs[1] : 0;
   out->solve_ms = ms;
   out->loop_ms = lms;
-  out->gpu_launches = launches + (max_cap > 0 && graph_mode ? hs[3] : 0) + (blocked ? 1 : 0);
+  out->gpu_launches = launches + (max_cap > 0 && graph_mode ? hs[3] : 0) + (blocked ? 1 : 0) + sum_launches;
   double rmax = 0.0;
   for (double r : *res) rmax = std::max(rmax, r);
   out->residual = rmax;

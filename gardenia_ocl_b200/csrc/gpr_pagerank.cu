@@ -415,18 +415,6 @@ __global__ void __launch_bounds__(NT, MINB) k_pr_blocked(PrArgs a) {
   }
 }
 
-// |s| summed per CTA: a grid of kSumBlocks CTAs always, so that the sum of `part` is the
-// same on every run.
-constexpr int kSumBlocks = 256;
-__global__ void __launch_bounds__(256) k_sum_abs(int m, const float *__restrict__ s,
-                                                 double *part) {
-  double t = 0.0;
-  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < m; i += kSumBlocks * 256LL)
-    t += (double)fabsf(s[i]);
-  t = block_sum(t);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
-}
-
 // Largest |score| (bits of a non-negative float order like the float; a NaN
 // sorts above every finite value and infinity).
 __global__ void k_max_abs(int m, const float *__restrict__ s, unsigned *out) {
@@ -791,7 +779,7 @@ int setup_blocked(gpr_graph *g, int sms) {
   g->max_grid = std::max(g->max_grid, g->grid_blocked);
   GPR_TRY(gpr::dalloc(&g->tq, 2, "tile queue"));
   GPR_TRY(gpr::dalloc(&g->fx_max, 1, "largest score"));
-  GPR_TRY(gpr::dalloc(&g->fx_part, kSumBlocks, "score sums"));
+  GPR_TRY(gpr::dalloc(&g->fx_part, gpr::kSumBlocks, "score sums"));
   return GPR_OK;
 }
 
@@ -991,28 +979,6 @@ int graph_loop(gpr_graph *g, const PrArgs &a, int ki, cudaStream_t st) {
 // score, or more mass than leaves enough bits); the caller solves another way.
 constexpr int kBlockedFallback = 100;
 
-// Fixed-point exponent S of the blocked form for a solve whose sweeps hold a total
-// |score| of at most b0 (a sweep maps total mass M to at most (1-d) + d*M, so the
-// larger of 1 and the initial mass bounds them all): a row's sum is at most that, so
-// |sum| * 2^S < 2^63 needs S <= 62 - log2(b0), blocked_cap.  Within that, S puts a
-// typical contribution (about b0 / nnz) near 2^28, so most fit the low 32-bit word of
-// the accumulator; S >= 31 unless b0 > 2^31.
-int blocked_cap(double b0) { return 62 - (int)ceil(log2(b0)); }
-
-int blocked_shift(long long nnz, double b0) {
-  const int pref = (int)floor(log2(std::max(1.0, (double)nnz) / b0)) + 28;
-  return std::min(blocked_cap(b0), std::max(31, pref));
-}
-
-// The S from which on the rounding to 2^-S is lost in a score's own FP32 rounding:
-// the roundings of a row of k contributions add up to about sqrt(k / 12) * 2^-S, and
-// no score of a sweep from scores >= 0 is below the base (1-d) / m.  With the mean
-// in-degree for k, that error is a quarter of 2^-24 of the base; rows of more
-// in-edges hold more than the base.  No S is enough for d = 1.
-double blocked_bits(int m, long long nnz, double d) {
-  return 24.0 + log2((double)m / (1.0 - d)) + 0.5 * log2(std::max(1.0, (double)nnz / m));
-}
-
 // One solve with sweep kernel ki (or, when `blocked`, the blocked form) from
 // the scores in d_scores (device, vertex order); the result is written back
 // to d_scores.
@@ -1084,24 +1050,26 @@ int solve_impl(gpr_graph *g, float *d_scores, const gpr_pr_opts &o, int ki, gpr_
     // earlier solution with its hubs), the mass itself is summed, and where that is
     // too large as well (all ones) the form does not apply.  A caller who asked for
     // the blocked form by name gets the S of the bound.
-    // Largest relative error against 64 bits, RMAT, 2^22 vertices, edge factor 16: S from
-    // the bound alone 1.8e-2 from one vertex and 7.8e-6 from an earlier solution, from
-    // the mass 2e-7 for both.
-    int S = blocked_shift(g->L.nnz, std::max(1.0, (double)m * (double)mx));
-    const double bits_needed = blocked_bits(m, g->L.nnz, (double)o.damping);
+    // Largest relative error against 64 bits after 25 sweeps, RMAT, 2^22 vertices, edge
+    // factor 16: S from the bound alone 1.7e-2 from one vertex, 9.9e-6 from an earlier
+    // solution and 4.8e-3 from all ones; from the mass 1.7e-7 for the first two, and the
+    // last in the exact order 5.6e-7, edge by edge (push) 1.4e-6.  3.6 ms a solve in blocks,
+    // 3.75 in the exact order, 9.8 edge by edge.
+    int S = gpr::blocked_shift(g->L.nnz, std::max(1.0, (double)m * (double)mx));
+    const double bits_needed = gpr::blocked_bits(m, g->L.nnz, (double)o.damping);
     if (o.form != GPR_FORM_BLOCKED && (double)S < bits_needed) {
-      std::vector<double> part(kSumBlocks);
-      k_sum_abs<<<kSumBlocks, 256, 0, st>>>(m, g->s, g->fx_part);
+      std::vector<double> part(gpr::kSumBlocks);
+      gpr::blk::k_sum_abs<<<gpr::kSumBlocks, 256, 0, st>>>(m, g->s, g->fx_part);
       ++launches;
       GPR_CUDA(cudaGetLastError());
-      GPR_CUDA(cudaMemcpyAsync(part.data(), g->fx_part, sizeof(double) * kSumBlocks,
+      GPR_CUDA(cudaMemcpyAsync(part.data(), g->fx_part, sizeof(double) * gpr::kSumBlocks,
                                cudaMemcpyDeviceToHost, st));
       GPR_CUDA(cudaStreamSynchronize(st));
       double mass = 0.0;
       for (double x : part) mass += x;
       const double b0 = std::max(1.0, mass * (1.0 + 1e-9));  // the sum's own rounding
-      if (bits_needed > (double)blocked_cap(b0)) return kBlockedFallback;
-      S = std::max(blocked_shift(g->L.nnz, b0), (int)ceil(bits_needed));
+      if (bits_needed > (double)gpr::blocked_cap(b0)) return kBlockedFallback;
+      S = std::max(gpr::blocked_shift(g->L.nnz, b0), (int)ceil(bits_needed));
     }
     a.fx_scale = ldexpf(1.f, S);
     a.fx_inv = ldexp(1.0, -S);

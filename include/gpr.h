@@ -255,7 +255,9 @@ int gpr_pagerank_push(gpr_graph *g, float *any_scores, const gpr_pr_opts *opts,
  * opts->form then works as for gpr_pagerank: BLOCKED sums every graph's rows
  * in 64-bit fixed point (one exponent S for the batch, from its edge count
  * and the largest m_g x |initial score|), FP32 and the persistent loop only;
- * AUTO picks it from 50,331,648 edges in the batch, else the units form.
+ * AUTO picks it from 50,331,648 edges in the batch, else the units form, and
+ * where that S would show in the scores takes one from the sum of the initial
+ * |scores| (see gpr_form) or, where that has no room, the units form.
  *
  * gpr_multigraph_pagerank solves every graph as gpr_pagerank would solve it
  * alone -- base (1 - kDamp) / m_g, its own L1 residual, stop after its first

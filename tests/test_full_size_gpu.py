@@ -66,6 +66,32 @@ def test_multigraph_512_sample_full_size(G, O):
         assert np.all(np.abs(s[a:b] - ref) <= 1e-6 + np.abs(ref - s64)), g
 
 
+@pytest.mark.parametrize("kind", ["one_vertex", "ones"])
+def test_multigraph_512_from_starts_far_from_uniform(G, O, kind):
+    """AUTO solves this batch in blocks from 1/m_g; from all of a graph's mass on one
+    vertex, and from all ones, each score is still within (8 + 4 sqrt(k)) 2^-24 of
+    the graph's FP64 recurrence (k in-edges; a few roundings, sqrt(k) for the sum)."""
+    A, voff = G.gen_multigraph(512, 1000, 500000, seed=1)
+    rp, col, od = A.rowptr.to_numpy(), A.col.to_numpy(), A.third.to_numpy()
+    assert A.nnz >= 50331648
+    s0 = np.ones(int(voff[-1]), dtype=np.float32)
+    if kind == "one_vertex":
+        s0[:] = 0.0
+        for a, b in zip(voff[:-1], voff[1:]):
+            s0[a + int(np.argmax(od[a:b]))] = 1.0
+    with G.MultiGraph(A.rowptr, A.col, A.third, voff, nnz=A.nnz, blocked=True) as mg:
+        s, iters, _, _ = mg.pagerank(s0.copy(), tol=0.0, max_iter=12)
+    A.close()
+    sizes = np.diff(voff)
+    for g in {int(np.argmax(sizes)), int(np.argmin(sizes)), 100, 101}:
+        a, b = int(voff[g]), int(voff[g + 1])
+        e0, e1 = int(rp[a]), int(rp[b])
+        lrp = rp[a:b + 1] - e0
+        ref, _, _ = O.pr_f64(lrp, col[e0:e1] - a, od[a:b], tol=0.0, max_iter=12, init=s0[a:b])
+        bound = (8 + 4 * np.sqrt(np.diff(lrp))) * 2.0 ** -24
+        assert iters[g] == 12 and np.all(np.abs(s[a:b] - ref) <= bound * ref), g
+
+
 def test_ppr_rmat22_full_size(G, O):
     csr = G.gen_rmat(22, 16, seed=1)
     rp, col, od = csr.rowptr.to_numpy(), csr.col.to_numpy(), csr.third.to_numpy()
