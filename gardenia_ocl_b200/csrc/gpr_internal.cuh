@@ -346,7 +346,9 @@ struct gpr_graph {
   gpr::BlockedLayout B;
   bool has_blocked = false, blocked_ok = false;
   bool has_push = false;       // B was built by the push solver (pull solves do not use it)
-  bool push_plain = false;     // B could not be built for the push solver
+  bool push_checked = false;   // the push solver has compared edges and out-degrees
+  bool push_plain = false;     // the push solver does not use B: more edges than an
+                               // out-degree says, or B could not be built
   int grid_blocked = 0, blocked_ctas = 1;  // blocked-form CTAs: total, per SM
   int blocked_carve = 0;       // shared-memory share of the SM for them, percent
   int *tq = nullptr;

@@ -19,8 +19,9 @@
 // 3888 us before and 233 / 360 / 932 / 1242 / 2089 us after, so it is used at all sizes,
 // from every start whose mass its fixed point holds to better than FP32 (solve_impl).
 //
-// Where that form does not apply (a non-finite score, too much mass, damping 1, no
-// scratch for its layout) the edges go one by one: the in-CSR's edges as a list sorted by source (relabelled ids,
+// Where that form does not apply (a non-finite score, too much mass, damping 1, a
+// vertex with more edges than its out-degree, no scratch for its layout) the edges go
+// one by one: the in-CSR's edges as a list sorted by source (relabelled ids,
 // built on first use), so each warp reads 32 consecutive edges -- equal work
 // for every warp, and the contribution loads of one warp fall on a few
 // neighbouring sources.  One persistent cooperative launch for all sweeps:

@@ -230,8 +230,9 @@ int gpr_ppr(gpr_graph *g, int k, const int *h_seeds, float *any_x,
  * contributions to their destinations' accumulators in shared memory, in 64-bit
  * fixed point whose rounding is below that of the FP32 scores: deterministic.
  * Where fixed point cannot hold them so (a non-finite initial score, more mass
- * than its 62 bits leave room for -- all ones on a large graph --, damping 1), or
- * without the scratch for that layout, edges sorted by source add one by one in
+ * than its 62 bits leave room for -- all ones on a large graph --, damping 1, a
+ * vertex with more edges than its out-degree says), or without the scratch for
+ * that layout, edges sorted by source add one by one in
  * FP32, and the last bits of the result vary from run to run.  opts->form and
  * opts->variant are not read.  The graph must be created with GPR_LAYOUT_PUSH
  * (or GPR_LAYOUT_BATCHED); FP32 only. */

@@ -143,3 +143,28 @@ def test_push_from_starts_far_from_uniform(G, O, kind):
     assert np.all(rel <= bound), (rel.max(), np.sort(rel / bound)[-3:])
     _, n, _ = O.pr_f64(rp, col, od, tol=1e-5, max_iter=200, init=s0)
     assert abs(st_t.iterations - n) <= 1
+
+
+def test_push_with_too_small_out_degrees(G, O):
+    """Out-degrees are the caller's.  Half of the edges' number lets the scores grow in
+    every sweep, past what fixed point holds (2^55 here), and 0 gives infinities:
+    both as the reference's recurrence has them."""
+    rp, col, od = O.rmat_graph(12, 16, seed=7)
+    m = len(rp) - 1
+    half = np.where(od > 1, od // 2, od).astype(np.int32)
+    with G.Graph(rp, col, half, push=True) as g:
+        s, st = g.pagerank_push(tol=0.0, max_iter=80)
+    ref, _, _ = O.pr_f64(rp, col, half, tol=0.0, max_iter=80)
+    assert ref.max() > 2.0 ** 40
+    # 80 sweeps of (8 + 4 sqrt(k)) 2^-24 per vertex, passed on from sweep to sweep
+    bound = 80 * (8 + 4 * np.sqrt(np.diff(rp).max())) * 2.0 ** -24
+    assert np.all(np.abs(s - ref) <= bound * ref)
+    none = od.copy()
+    none[int(np.argmax(od))] = 0
+    with G.Graph(rp, col, none, push=True) as g:
+        s, st = g.pagerank_push(tol=0.0, max_iter=2)
+    ref, _, _ = O.pr_plain_f32(rp, col, none, tol=0.0, max_iter=2)
+    fin = np.isfinite(ref)
+    assert 0 < np.count_nonzero(fin) < m
+    assert np.array_equal(fin, np.isfinite(s))
+    assert np.abs(s[fin] - ref[fin]).max() <= 1e-6
