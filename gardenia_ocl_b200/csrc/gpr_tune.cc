@@ -15,8 +15,9 @@
 // the chosen form's knobs: for the exact order the kernel variant, hot
 // prefix, lanes-per-row bound and chunk threshold / size; for the blocked
 // form the rows per block, words per tile and the in-degree above which
-// rows are summed in chunks rather than in blocks.  Each candidate is timed as the best of kReps solves of exactly
-// `sweeps` sweeps (tol 0), device time of the sweep loop
+// rows are summed in chunks rather than in blocks.  The first candidate is the
+// library's own default layout.  Each candidate is timed as the best of kReps solves
+// of exactly `sweeps` sweeps (tol 0), device time of the sweep loop
 // (gpr_pr_stats.loop_ms), and taken only when at least kMargin faster than the
 // current pick.  The batch tuner first tries the blocked form for the whole
 // batch (with its rows per block and words per tile); otherwise it groups
@@ -25,7 +26,7 @@
 //
 // Cache file: one line per entry, later lines override earlier ones:
 //   <signature> <sell_max> <chunk> <chunk_min> <hot_entries> <variant> <ms_per_sweep>
-//       [<flags> <block_rows> <tile_words> [<blocked_long>]]
+//       [<flags> <block_rows> <tile_words> [<blocked_long> [<format>]]]
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
@@ -42,11 +43,15 @@
 namespace {
 
 constexpr int kReps = 3;
-constexpr int kDefSell = 64, kDefChunk = 4096, kDefChunkMin = 4096, kDefHot = 32768;
+constexpr int kDefSell = 64;
+// Last field of a cache line.  Lines without it hold a chunk of 4096 and a prefix of
+// 32768 entries where no candidate beat the defaults, which were these for every size.
+constexpr int kCacheFormat = 2;
 
+// 0: the library's default for the graph's size (a layout made without a tuner has
+// exactly these, so the first candidate is what a pick has to beat).
 struct Cfg {
-  int sell_max = kDefSell, chunk = kDefChunk, chunk_min = kDefChunkMin, hot = kDefHot,
-      variant = 0;
+  int sell_max = kDefSell, chunk = 0, chunk_min = 0, hot = 0, variant = 0;
   // blocked form (0: library defaults)
   int flags = 0, block_rows = 0, tile_words = 0, blocked_long = 0;
   bool operator==(const Cfg &o) const {
@@ -85,10 +90,13 @@ std::map<std::string, std::pair<Cfg, double>> load_cache(const char *path) {
     char key[128];
     Cfg x;
     double ms = 0;
-    const int n = sscanf(line, "%127s %d %d %d %d %d %lf %d %d %d %d", key, &x.sell_max, &x.chunk,
-                         &x.chunk_min, &x.hot, &x.variant, &ms, &x.flags, &x.block_rows,
-                         &x.tile_words, &x.blocked_long);
-    if (n == 7 || n == 10 || n == 11) c[key] = {x, ms};
+    int format = 1;
+    const int n = sscanf(line, "%127s %d %d %d %d %d %lf %d %d %d %d %d", key, &x.sell_max,
+                         &x.chunk, &x.chunk_min, &x.hot, &x.variant, &ms, &x.flags, &x.block_rows,
+                         &x.tile_words, &x.blocked_long, &format);
+    if (format < kCacheFormat && x.chunk == 4096 && x.chunk_min == 4096) x.chunk = x.chunk_min = 0;
+    if (format < kCacheFormat && x.hot == 32768) x.hot = 0;
+    if (n == 7 || n >= 10) c[key] = {x, ms};
   }
   fclose(f);
   return c;
@@ -98,8 +106,9 @@ void save_cache(const char *path, const std::string &key, const Cfg &x, double m
   if (!path) return;
   FILE *f = fopen(path, "a");
   if (!f) return;
-  fprintf(f, "%s %d %d %d %d %d %.6f %d %d %d %d\n", key.c_str(), x.sell_max, x.chunk,
-          x.chunk_min, x.hot, x.variant, ms, x.flags, x.block_rows, x.tile_words, x.blocked_long);
+  fprintf(f, "%s %d %d %d %d %d %.6f %d %d %d %d %d\n", key.c_str(), x.sell_max, x.chunk,
+          x.chunk_min, x.hot, x.variant, ms, x.flags, x.block_rows, x.tile_words, x.blocked_long,
+          kCacheFormat);
   fclose(f);
 }
 
@@ -176,6 +185,10 @@ struct SingleBench {
 // A candidate must beat the current pick by this fraction to replace it, so
 // run-to-run timing noise does not move the pick.
 constexpr double kMargin = 0.03;
+
+// Candidate (chunk_min, chunk) pairs.
+const std::vector<std::pair<int, int>> kChunkPairs = {{512, 512},   {1024, 1024},  {2048, 2048},
+                                                      {4096, 4096}, {16384, 4096}, {4096, 1024}};
 
 // Coordinate descent over one knob: keeps the best of `vals` applied to x.
 template <typename F, typename T>
@@ -258,12 +271,11 @@ int gpr_tune_graph(int m, long long nnz, const int *any_rowptr, const int *any_c
   } else {
     descend(&x, &best, std::vector<int>{1, 2, 3, 4, 5, 6, 7},
             [](Cfg *y, int v) { y->variant = v; }, time);
-    descend(&x, &best, std::vector<int>{8192, 16384, 56832},
+    descend(&x, &best, std::vector<int>{4096, 8192, 16384, 32768, 56832},
             [](Cfg *y, int v) { y->hot = v; }, time);
     descend(&x, &best, std::vector<int>{16, 32, 128}, [](Cfg *y, int v) { y->sell_max = v; },
             time);
-    descend(&x, &best,
-            std::vector<std::pair<int, int>>{{1024, 1024}, {16384, 4096}, {4096, 1024}},
+    descend(&x, &best, kChunkPairs,
             [](Cfg *y, std::pair<int, int> v) {
               y->chunk_min = v.first;
               y->chunk = v.second;
@@ -380,7 +392,7 @@ int gpr_tune_multigraph(int n_graphs, const int *h_voff, long long nnz, const in
     };
     Cfg x = pick[k];
     descend(&x, &best, std::vector<int>{16, 32, 128}, [](Cfg *y, int v) { y->sell_max = v; }, time);
-    descend(&x, &best, std::vector<std::pair<int, int>>{{1024, 1024}, {16384, 4096}, {4096, 1024}},
+    descend(&x, &best, kChunkPairs,
             [](Cfg *y, std::pair<int, int> v) {
               y->chunk_min = v.first;
               y->chunk = v.second;

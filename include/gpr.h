@@ -298,7 +298,8 @@ int gpr_multigraph_pagerank(gpr_multigraph *mg, float *any_scores,
  * `sweeps` sweeps after a warm-up solve, kept only when 3% faster than the
  * current pick), and caches the pick per distribution signature in the text
  * file cache_path (NULL: no cache).  A cached signature returns at once
- * (from_cache = 1). */
+ * (from_cache = 1).  The first candidate is the default layout; where a default
+ * stays the pick, the layout's field is 0. */
 typedef struct {
   gpr_layout_opts layout;       /* pass to gpr_graph_create_ex */
   int variant;                  /* pass as gpr_pr_opts.variant */

@@ -1,10 +1,12 @@
 """Autotuner: distribution signatures and the cache (CPU), the search on the
 GPU (the pick must solve to the same answer as the defaults)."""
 import os
+import subprocess
 
 import numpy as np
 import pytest
 
+from conftest import ROOT
 from graphs import erdos_renyi, star
 
 LAYOUT_KEYS = ("sell_max", "chunk", "chunk_min", "hot_entries", "blocked", "block_rows",
@@ -46,6 +48,71 @@ def test_cache_entries_of_the_blocked_form(G, tmp_path):
     assert r["blocked_long"] == 0  # ten-field lines: the library default
     r = G.tune_cache_lookup(p, "pr:m22:d4:s2")
     assert r["blocked"] and r["blocked_long"] == 16384 and r["block_rows"] == 0
+
+
+@pytest.fixture(scope="module")
+def driver(tmp_path_factory):
+    """gpr_tune.cc over a library that only keeps books (tune_driver.cc)."""
+    out = str(tmp_path_factory.mktemp("tune") / "tune_driver")
+    csrc = os.path.join(ROOT, "gardenia_ocl_b200", "csrc")
+    subprocess.run(["/usr/bin/g++", "-std=c++17", "-O1", "-o", out,
+                    os.path.join(ROOT, "tests", "tune_driver.cc"), os.path.join(csrc, "gpr_tune.cc"),
+                    "-I", os.path.join(ROOT, "include"), "-I", csrc], check=True)
+
+    def run(kind, chunk, hot, cache):
+        p = subprocess.run([out, kind, str(chunk), str(hot), str(cache)], capture_output=True,
+                           text=True, timeout=60)
+        assert p.returncode == 0, p.stderr
+        lines = [l.split() for l in p.stdout.splitlines()]
+        pick = [l for l in lines if l[0] == "pick"][0]
+        ms = [l for l in lines if l[0] == "ms"][0]
+        return ([tuple(map(int, l[1:])) for l in lines if l[0] == "create"],
+                tuple(map(int, pick[1:])), float(ms[1]), float(ms[2]), int(ms[4]))
+
+    return run
+
+
+@pytest.mark.parametrize("kind", ["single", "batch"])
+def test_search_starts_from_the_library_defaults(driver, tmp_path, kind):
+    """The first candidate leaves chunk, chunk_min and hot_entries to the library, as a
+    graph made without a tuner does; where nothing is faster that is the pick, and
+    it comes back from the cache so."""
+    cache = tmp_path / "tune.txt"
+    made, pick, ms, ms0, cached = driver(kind, 0, 0, cache)
+    assert made[0] == (64, 0, 0, 0, 0)
+    assert pick == (64, 0, 0, 0, 0) and ms == ms0 == 10.0 and not cached
+    made, pick, ms, _, cached = driver(kind, 0, 0, cache)
+    assert len(made) == (0 if kind == "single" else 1)
+    assert pick == (64, 0, 0, 0, 0) and ms == 10.0
+
+
+@pytest.mark.parametrize("chunk", [512, 1024, 2048, 4096])
+@pytest.mark.parametrize("hot", [4096, 16384, 32768])
+def test_search_finds_the_fastest_bins(driver, tmp_path, chunk, hot):
+    cache = tmp_path / "tune.txt"
+    _, pick, ms, ms0, _ = driver("single", chunk, hot, cache)
+    assert pick == (64, chunk, chunk, hot, 0) and ms == 6.0 and ms0 == 10.0
+    made, pick, ms, _, cached = driver("single", chunk, hot, cache)
+    assert not made and cached and pick == (64, chunk, chunk, hot, 0)
+    _, pick, ms, _, _ = driver("batch", chunk, 0, tmp_path / "batch.txt")
+    assert pick == (64, chunk, chunk, 0, 0) and ms == 8.0
+
+
+def test_cache_entries_of_the_fixed_defaults(G, tmp_path):
+    """Lines without a format number come from a tuner that gave its defaults, a chunk
+    of 4096 and a prefix of 32768 for every size, explicitly: they stand for the
+    library's defaults.  With the number they are picks."""
+    p = str(tmp_path / "tune.txt")
+    with open(p, "w") as f:
+        f.write("pr:m16:d4:s2 64 4096 4096 32768 2 0.5\n")
+        f.write("pr:m17:d4:s2 64 4096 16384 8192 2 0.5 0 0 0 0\n")
+        f.write("pr:m18:d4:s2 64 4096 4096 32768 2 0.5 0 0 0 0 2\n")
+    r = G.tune_cache_lookup(p, "pr:m16:d4:s2")
+    assert (r["chunk"], r["chunk_min"], r["hot_entries"], r["variant"]) == (0, 0, 0, 2)
+    r = G.tune_cache_lookup(p, "pr:m17:d4:s2")
+    assert (r["chunk"], r["chunk_min"], r["hot_entries"]) == (4096, 16384, 8192)
+    r = G.tune_cache_lookup(p, "pr:m18:d4:s2")
+    assert (r["chunk"], r["chunk_min"], r["hot_entries"]) == (4096, 4096, 32768)
 
 
 @pytest.mark.gpu
