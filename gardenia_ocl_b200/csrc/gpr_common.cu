@@ -1,12 +1,9 @@
-// Error slot, allocation helpers and small C-ABI entry points.
+// Error slot, copy helpers and small C-ABI entry points.
 #include <cub/cub.cuh>
 #include <stdarg.h>
 #include <string.h>
 
 #include <algorithm>
-#include <mutex>
-#include <unordered_map>
-#include <vector>
 
 #include "gpr_internal.cuh"
 
@@ -19,199 +16,6 @@ void set_error(const char *fmt, ...) {
   va_start(ap, fmt);
   vsnprintf(g_err, sizeof(g_err), fmt, ap);
   va_end(ap);
-}
-
-// Block cache of device allocations.  One-shot solver calls (the reference's
-// PRSolver shape: copy in, build, solve, free) make dozens of allocations each, of
-// a few bytes to gigabytes: mapping and unmapping the large ones makes cudaMalloc
-// / cudaFree slow and erratic, and every cudaFree of a small one waits for the
-// device.  Blocks are kept after dfree and handed out again: large ones (kCacheMin
-// bytes and more) to requests that fit them within 1/8, at most kCacheCap bytes of
-// them; small ones by size class (powers of two from kSmallMin), at most kSmallCap
-// bytes.  A freed block may still be in use by a kernel, so it is handed out again
-// only behind a device synchronisation: one when the first block freed since the
-// last one is taken, for all of them.  An allocation that fails releases the
-// cache and retries; gpr_release_cached() empties it.
-// One-shot PageRank of 65,536 vertices on host arrays: 2.76 ms with the small blocks
-// allocated and freed each time and a synchronisation per free, 1.20 ms this way.
-namespace {
-
-constexpr size_t kCacheMin = size_t(1) << 20;
-constexpr size_t kCacheCap = size_t(24) << 30;
-constexpr size_t kSmallMin = 512;
-constexpr size_t kSmallCap = size_t(64) << 20;
-constexpr int kSmallClasses = 11;  // 512 bytes .. 512 KiB
-
-struct Block {
-  void *p;
-  size_t bytes;
-  int device;
-  unsigned long long freed;  // number of the free (g_frees) that returned it
-};
-
-std::mutex g_mu;
-std::unordered_map<void *, Block> g_live;  // blocks handed out
-std::vector<Block> g_free;                // cached large blocks, unused
-std::vector<Block> g_small[kSmallClasses];  // cached small blocks, by class
-size_t g_free_bytes = 0, g_small_bytes = 0;
-unsigned long long g_frees = 0;
-std::unordered_map<int, unsigned long long> g_synced;  // per device: frees it has waited for
-
-int small_class(size_t bytes) {
-  int c = 0;
-  while ((kSmallMin << c) < bytes) ++c;
-  return c;
-}
-
-void give_back(const Block &b) {
-  int cur = -1;
-  cudaGetDevice(&cur);
-  if (cur != b.device) cudaSetDevice(b.device);
-  cudaFree(b.p);
-  if (cur >= 0 && cur != b.device) cudaSetDevice(cur);
-}
-
-void release_free_locked(int device) {
-  auto drop = [&](std::vector<Block> &v, size_t &total) {
-    for (size_t i = 0; i < v.size();) {
-      if (device < 0 || v[i].device == device) {
-        give_back(v[i]);
-        total -= v[i].bytes;
-        v[i] = v.back();
-        v.pop_back();
-      } else {
-        ++i;
-      }
-    }
-  };
-  drop(g_free, g_free_bytes);
-  for (auto &v : g_small) drop(v, g_small_bytes);
-}
-
-// Takes entry i of a free list for the current device `dev`.
-void *take_locked(std::vector<Block> &v, size_t i, size_t &total, int dev) {
-  Block b = v[i];
-  v[i] = v.back();
-  v.pop_back();
-  total -= b.bytes;
-  unsigned long long &synced = g_synced[dev];
-  if (b.freed > synced) {
-    cudaDeviceSynchronize();
-    synced = g_frees;
-  }
-  g_live[b.p] = b;
-  return b.p;
-}
-
-}  // namespace
-
-int dmalloc(void **p, size_t bytes, const char *what) {
-  *p = nullptr;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (bytes > (kSmallMin << (kSmallClasses - 1)) && bytes < kCacheMin) bytes = kCacheMin;
-  if (bytes >= kCacheMin) {
-    std::lock_guard<std::mutex> lk(g_mu);
-    int best = -1;
-    for (size_t i = 0; i < g_free.size(); ++i) {
-      const Block &b = g_free[i];
-      if (b.device == dev && b.bytes >= bytes && b.bytes - bytes <= bytes / 8 &&
-          (best < 0 || b.bytes < g_free[best].bytes))
-        best = (int)i;
-    }
-    if (best >= 0) {
-      *p = take_locked(g_free, (size_t)best, g_free_bytes, dev);
-      return GPR_OK;
-    }
-  } else {
-    const int c = small_class(bytes);
-    bytes = kSmallMin << c;
-    std::lock_guard<std::mutex> lk(g_mu);
-    std::vector<Block> &v = g_small[c];
-    for (size_t i = v.size(); i-- > 0;)
-      if (v[i].device == dev) {
-        *p = take_locked(v, i, g_small_bytes, dev);
-        return GPR_OK;
-      }
-  }
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    {
-      std::lock_guard<std::mutex> lk(g_mu);
-      release_free_locked(dev);
-    }
-    e = cudaMalloc(p, bytes);
-  }
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    *p = nullptr;
-    set_error("cudaMalloc(%zu bytes) for %s: out of device memory", bytes, what);
-    return GPR_ENOMEM;
-  }
-  if (e != cudaSuccess) {
-    *p = nullptr;
-    set_error("cudaMalloc(%zu bytes) for %s: %s", bytes, what, cudaGetErrorString(e));
-    return GPR_ECUDA;
-  }
-  std::lock_guard<std::mutex> lk(g_mu);
-  g_live[*p] = Block{*p, bytes, dev, 0};
-  return GPR_OK;
-}
-
-namespace {
-thread_local std::vector<void *> *t_deferred = nullptr;
-}  // namespace
-
-DeferFrees::DeferFrees() : prev_(t_deferred) { t_deferred = &list_; }
-
-DeferFrees::~DeferFrees() {
-  t_deferred = prev_;
-  for (void *p : list_) dfree(p);
-}
-
-void dfree(void *p) {
-  if (!p) return;
-  if (t_deferred) {
-    t_deferred->push_back(p);
-    return;
-  }
-  std::unique_lock<std::mutex> lk(g_mu);
-  auto it = g_live.find(p);
-  if (it == g_live.end()) {
-    lk.unlock();
-    cudaFree(p);
-    return;
-  }
-  Block b = it->second;
-  g_live.erase(it);
-  b.freed = ++g_frees;
-  if (b.bytes < kCacheMin) {
-    if (g_small_bytes + b.bytes > kSmallCap) {
-      give_back(b);
-      return;
-    }
-    g_small_bytes += b.bytes;
-    g_small[small_class(b.bytes)].push_back(b);
-    return;
-  }
-  g_free.push_back(b);
-  g_free_bytes += b.bytes;
-  while (g_free_bytes > kCacheCap && !g_free.empty()) {
-    size_t big = 0;
-    for (size_t i = 1; i < g_free.size(); ++i)
-      if (g_free[i].bytes > g_free[big].bytes) big = i;
-    Block v = g_free[big];
-    g_free[big] = g_free.back();
-    g_free.pop_back();
-    g_free_bytes -= v.bytes;
-    give_back(v);
-  }
-}
-
-size_t cached_bytes() {
-  std::lock_guard<std::mutex> lk(g_mu);
-  return g_free_bytes + g_small_bytes;
 }
 
 namespace {
@@ -348,40 +152,6 @@ int gpr_pr_opts_default(gpr_pr_opts *o) {
   o->refine_max = 64;
   o->ppr_repack = 1;
   return GPR_OK;
-}
-
-int gpr_free(void *d_ptr) {
-  if (d_ptr) GPR_CUDA(cudaDeviceSynchronize());  // as cudaFree: the caller's work on it is over
-  gpr::dfree(d_ptr);
-  GPR_CUDA(cudaGetLastError());
-  return GPR_OK;
-}
-
-int gpr_release_cached(long long *released_bytes) {
-  {
-    std::lock_guard<std::mutex> lk(gpr::g_mu);
-    if (released_bytes) *released_bytes = (long long)(gpr::g_free_bytes + gpr::g_small_bytes);
-    gpr::release_free_locked(-1);
-  }
-  GPR_CUDA(cudaGetLastError());
-  return GPR_OK;
-}
-
-int gpr_cached_bytes(long long *bytes) {
-  if (!bytes) {
-    gpr::set_error("gpr_cached_bytes: NULL out");
-    return GPR_EINVAL;
-  }
-  *bytes = (long long)gpr::cached_bytes();
-  return GPR_OK;
-}
-
-int gpr_malloc(void **d_ptr, size_t bytes) {
-  if (!d_ptr) {
-    gpr::set_error("gpr_malloc: NULL out");
-    return GPR_EINVAL;
-  }
-  return gpr::dmalloc(d_ptr, bytes ? bytes : 1, "gpr_malloc");
 }
 
 int gpr_memcpy(void *dst, const void *src, size_t bytes) {
