@@ -16,7 +16,8 @@ namespace gpr {
 // them; small ones by size class (powers of two from kSmallMin), at most kSmallCap
 // bytes.  A freed block may still be in use by a kernel, so it is handed out again
 // only behind a device synchronisation: one when the first block freed since the
-// last one is taken, for all of them.  An allocation that fails releases the
+// last one is taken, for all of them.  Where that is refused, a new block is
+// allocated.  An allocation that fails releases the
 // cache and retries; gpr_release_cached() empties it.
 // One-shot PageRank of 65,536 vertices on host arrays: 2.76 ms with the small blocks
 // allocated and freed each time and a synchronisation per free, 1.20 ms this way.
@@ -74,17 +75,22 @@ void release_free_locked(int device) {
   for (auto &v : g_small) drop(v, g_small_bytes);
 }
 
-// Takes entry i of a free list for the current device `dev`.
+// Takes entry i of a free list for the current device `dev`; null when the block may
+// still be in use and the wait for the device is refused (another thread captures a
+// stream): the block stays where it is.
 void *take_locked(std::vector<Block> &v, size_t i, size_t &total, int dev) {
   Block b = v[i];
+  unsigned long long &synced = g_synced[dev];
+  if (b.freed > synced) {
+    if (cudaDeviceSynchronize() != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    synced = g_frees;
+  }
   v[i] = v.back();
   v.pop_back();
   total -= b.bytes;
-  unsigned long long &synced = g_synced[dev];
-  if (b.freed > synced) {
-    cudaDeviceSynchronize();
-    synced = g_frees;
-  }
   g_live[b.p] = b;
   return b.p;
 }
@@ -107,7 +113,7 @@ int dmalloc(void **p, size_t bytes, const char *what) {
     }
     if (best >= 0) {
       *p = take_locked(g_free, (size_t)best, g_free_bytes, dev);
-      return GPR_OK;
+      if (*p) return GPR_OK;
     }
   } else {
     const int c = small_class(bytes);
@@ -117,7 +123,8 @@ int dmalloc(void **p, size_t bytes, const char *what) {
     for (size_t i = v.size(); i-- > 0;)
       if (v[i].device == dev) {
         *p = take_locked(v, i, g_small_bytes, dev);
-        return GPR_OK;
+        if (*p) return GPR_OK;
+        break;
       }
   }
   cudaError_t e = cudaMalloc(p, bytes);
