@@ -58,11 +58,13 @@ void give_back(const Block &b) {
   if (cur >= 0 && cur != b.device) cudaSetDevice(cur);
 }
 
-void release_free_locked(int device) {
+// Takes the cached blocks of a device (-1: of all) out of the cache.
+std::vector<Block> drain_locked(int device) {
+  std::vector<Block> out;
   auto drop = [&](std::vector<Block> &v, size_t &total) {
     for (size_t i = 0; i < v.size();) {
       if (device < 0 || v[i].device == device) {
-        give_back(v[i]);
+        out.push_back(v[i]);
         total -= v[i].bytes;
         v[i] = v.back();
         v.pop_back();
@@ -73,24 +75,58 @@ void release_free_locked(int device) {
   };
   drop(g_free, g_free_bytes);
   for (auto &v : g_small) drop(v, g_small_bytes);
+  return out;
 }
 
-// Takes entry i of a free list for the current device `dev`; null when the block may
-// still be in use and the wait for the device is refused (another thread captures a
-// stream): the block stays where it is.
-void *take_locked(std::vector<Block> &v, size_t i, size_t &total, int dev) {
-  Block b = v[i];
-  unsigned long long &synced = g_synced[dev];
-  if (b.freed > synced) {
-    if (cudaDeviceSynchronize() != cudaSuccess) {
-      cudaGetLastError();
+// Cached block for a request on device `dev`: the smallest large block that holds
+// `bytes` within 1/8, or the last small block of its class, out of its list.
+bool find_locked(size_t bytes, int dev, Block *out) {
+  std::vector<Block> &v = bytes >= kCacheMin ? g_free : g_small[small_class(bytes)];
+  int best = -1;
+  for (size_t i = v.size(); i-- > 0;) {
+    const Block &b = v[i];
+    if (b.device != dev || b.bytes < bytes || b.bytes - bytes > bytes / 8) continue;
+    if (best < 0 || b.bytes < v[best].bytes) best = (int)i;
+    if (bytes < kCacheMin) break;
+  }
+  if (best < 0) return false;
+  *out = v[best];
+  v[best] = v.back();
+  v.pop_back();
+  (bytes >= kCacheMin ? g_free_bytes : g_small_bytes) -= out->bytes;
+  return true;
+}
+
+void put_locked(const Block &b) {
+  if (b.bytes >= kCacheMin) {
+    g_free.push_back(b);
+    g_free_bytes += b.bytes;
+  } else {
+    g_small[small_class(b.bytes)].push_back(b);
+    g_small_bytes += b.bytes;
+  }
+}
+
+// A cached block for the current device `dev`, or null.  The wait for the device is
+// made without the lock, so that other threads allocate and free meanwhile; it covers
+// the blocks freed before it.  Where it is refused (another thread captures a stream)
+// the block goes back.
+void *take(size_t bytes, int dev) {
+  std::unique_lock<std::mutex> lk(g_mu);
+  Block b;
+  if (!find_locked(bytes, dev, &b)) return nullptr;
+  if (b.freed > g_synced[dev]) {
+    const unsigned long long upto = g_frees;
+    lk.unlock();
+    const cudaError_t e = cudaDeviceSynchronize();
+    if (e != cudaSuccess) cudaGetLastError();
+    lk.lock();
+    if (e != cudaSuccess) {
+      put_locked(b);
       return nullptr;
     }
-    synced = g_frees;
+    if (g_synced[dev] < upto) g_synced[dev] = upto;
   }
-  v[i] = v.back();
-  v.pop_back();
-  total -= b.bytes;
   g_live[b.p] = b;
   return b.p;
 }
@@ -102,38 +138,18 @@ int dmalloc(void **p, size_t bytes, const char *what) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (bytes > (kSmallMin << (kSmallClasses - 1)) && bytes < kCacheMin) bytes = kCacheMin;
-  if (bytes >= kCacheMin) {
-    std::lock_guard<std::mutex> lk(g_mu);
-    int best = -1;
-    for (size_t i = 0; i < g_free.size(); ++i) {
-      const Block &b = g_free[i];
-      if (b.device == dev && b.bytes >= bytes && b.bytes - bytes <= bytes / 8 &&
-          (best < 0 || b.bytes < g_free[best].bytes))
-        best = (int)i;
-    }
-    if (best >= 0) {
-      *p = take_locked(g_free, (size_t)best, g_free_bytes, dev);
-      if (*p) return GPR_OK;
-    }
-  } else {
-    const int c = small_class(bytes);
-    bytes = kSmallMin << c;
-    std::lock_guard<std::mutex> lk(g_mu);
-    std::vector<Block> &v = g_small[c];
-    for (size_t i = v.size(); i-- > 0;)
-      if (v[i].device == dev) {
-        *p = take_locked(v, i, g_small_bytes, dev);
-        if (*p) return GPR_OK;
-        break;
-      }
-  }
+  if (bytes < kCacheMin) bytes = kSmallMin << small_class(bytes);
+  *p = take(bytes, dev);
+  if (*p) return GPR_OK;
   cudaError_t e = cudaMalloc(p, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
+    std::vector<Block> kept;
     {
       std::lock_guard<std::mutex> lk(g_mu);
-      release_free_locked(dev);
+      kept = drain_locked(dev);
     }
+    for (const Block &b : kept) give_back(b);
     e = cudaMalloc(p, bytes);
   }
   if (e == cudaErrorMemoryAllocation) {
@@ -179,17 +195,12 @@ void dfree(void *p) {
   Block b = it->second;
   g_live.erase(it);
   b.freed = ++g_frees;
-  if (b.bytes < kCacheMin) {
-    if (g_small_bytes + b.bytes > kSmallCap) {
-      give_back(b);
-      return;
-    }
-    g_small_bytes += b.bytes;
-    g_small[small_class(b.bytes)].push_back(b);
+  if (b.bytes < kCacheMin && g_small_bytes + b.bytes > kSmallCap) {
+    lk.unlock();
+    give_back(b);
     return;
   }
-  g_free.push_back(b);
-  g_free_bytes += b.bytes;
+  put_locked(b);
   while (g_free_bytes > kCacheCap && !g_free.empty()) {
     size_t big = 0;
     for (size_t i = 1; i < g_free.size(); ++i)
@@ -198,7 +209,9 @@ void dfree(void *p) {
     g_free[big] = g_free.back();
     g_free.pop_back();
     g_free_bytes -= v.bytes;
+    lk.unlock();  // cudaFree waits for the device
     give_back(v);
+    lk.lock();
   }
 }
 
@@ -219,11 +232,13 @@ int gpr_free(void *d_ptr) {
 }
 
 int gpr_release_cached(long long *released_bytes) {
+  std::vector<gpr::Block> kept;
   {
     std::lock_guard<std::mutex> lk(gpr::g_mu);
     if (released_bytes) *released_bytes = (long long)(gpr::g_free_bytes + gpr::g_small_bytes);
-    gpr::release_free_locked(-1);
+    kept = gpr::drain_locked(-1);
   }
+  for (const gpr::Block &b : kept) gpr::give_back(b);
   GPR_CUDA(cudaGetLastError());
   return GPR_OK;
 }

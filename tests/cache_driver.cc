@@ -113,34 +113,32 @@ void refused() {
 }
 
 // While one thread waits for the GPU, others allocate and free.
-bool other_done = false;
+bool in_wait = false, other_done = false;
 void while_waiting() {
   std::unique_lock<std::mutex> lk(mu);
+  in_wait = true;
   cv.notify_all();
   expect(cv.wait_for(lk, std::chrono::seconds(5), [] { return other_done; }),
          "another thread's allocation and free do not wait for the GPU");
 }
-void threads(void (*waiter)(void *)) {
+void waiting_in_malloc() {
   void *a = get(1000), *b = get(2000);
   gpr::dfree(a);
   on_sync = while_waiting;
   std::thread other([&] {
     {
       std::unique_lock<std::mutex> lk(mu);
-      cv.wait_for(lk, std::chrono::seconds(5));
+      cv.wait(lk, [] { return in_wait; });
+      on_sync = nullptr;
     }
-    on_sync = nullptr;
     gpr::dfree(get(5000));
     gpr::dfree(b);
     std::lock_guard<std::mutex> lk(mu);
     other_done = true;
     cv.notify_all();
   });
-  waiter(a);
+  expect(get(1000) == a, "the block behind the wait");
   other.join();
-}
-void waiting_in_malloc() {
-  threads([](void *a) { expect(get(1000) == a, "the block behind the wait"); });
   // blocks freed during that wait are not covered by it
   const size_t before = syncs.size();
   get(2000);

@@ -32,3 +32,7 @@ def test_one_wait_for_all_blocks_freed_before(driver):
 
 def test_a_refused_wait_hands_out_nothing(driver):
     assert driver("refused") == "ok\n"
+
+
+def test_other_threads_go_on_while_one_waits(driver):
+    assert driver("threads") == "ok\n"
