@@ -58,6 +58,22 @@ void give_back(const Block &b) {
   if (cur >= 0 && cur != b.device) cudaSetDevice(cur);
 }
 
+// Waits for the device of a block that is handed out (others are left to cudaFree).
+cudaError_t wait_for_owner(void *p) {
+  int device = -1, cur = -1;
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_live.find(p);
+    if (it == g_live.end()) return cudaSuccess;
+    device = it->second.device;
+  }
+  cudaGetDevice(&cur);
+  if (cur != device) cudaSetDevice(device);
+  const cudaError_t e = cudaDeviceSynchronize();
+  if (cur >= 0 && cur != device) cudaSetDevice(cur);
+  return e;
+}
+
 // Takes the cached blocks of a device (-1: of all) out of the cache.
 std::vector<Block> drain_locked(int device) {
   std::vector<Block> out;
@@ -225,8 +241,11 @@ size_t cached_bytes() {
 extern "C" {
 
 int gpr_free(void *d_ptr) {
-  if (d_ptr) GPR_CUDA(cudaDeviceSynchronize());  // as cudaFree: the caller's work on it is over
+  // As cudaFree, waits for the device of the block, so that the caller's work on it is
+  // over, and frees it whatever that work's status.
+  const cudaError_t e = gpr::wait_for_owner(d_ptr);
   gpr::dfree(d_ptr);
+  GPR_CUDA(e);
   GPR_CUDA(cudaGetLastError());
   return GPR_OK;
 }

@@ -36,3 +36,7 @@ def test_a_refused_wait_hands_out_nothing(driver):
 
 def test_other_threads_go_on_while_one_waits(driver):
     assert driver("threads") == "ok\n"
+
+
+def test_gpr_free_waits_for_the_device_of_the_block(driver):
+    assert driver("free") == "ok\n"
