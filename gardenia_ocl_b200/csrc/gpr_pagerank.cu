@@ -705,6 +705,17 @@ PrArgs make_args(gpr_graph *g, const gpr_pr_opts &o, int ki) {
 
 void drop_loop_graph(gpr_graph *g);
 
+// The blocked layout and the buffers of setup_blocked.
+void drop_blocked(gpr_graph *g) {
+  gpr::free_blocked_layout(&g->B);
+  gpr::dfree(g->tq);
+  gpr::dfree(g->fx_max);
+  gpr::dfree(g->fx_part);
+  g->tq = nullptr;
+  g->fx_max = nullptr;
+  g->fx_part = nullptr;
+}
+
 void destroy(gpr_graph *g) {
   if (!g) return;
   drop_loop_graph(g);
@@ -731,10 +742,7 @@ void destroy(gpr_graph *g) {
   gpr::dfree(g->push_src);
   gpr::dfree(g->push_dst);
   gpr::dfree(g->push_sum);
-  gpr::free_blocked_layout(&g->B);
-  gpr::dfree(g->tq);
-  gpr::dfree(g->fx_max);
-  gpr::dfree(g->fx_part);
+  drop_blocked(g);
   if (g->e0) cudaEventDestroy(g->e0);
   if (g->e1) cudaEventDestroy(g->e1);
   if (g->e2) cudaEventDestroy(g->e2);
@@ -1329,10 +1337,9 @@ int build_push_layout(gpr_graph *g) {
                                    gpr::kTileWordsDefault, gpr::kRunWords,
                                    sms * gpr::blocked_ctas_per_sm(R), &g->B, g->st);
   gpr::dfree(perm);
-  GPR_TRY(rc);
   const int grid = g->max_grid;
   double *part = nullptr;
-  rc = setup_blocked(g, sms);
+  if (rc == GPR_OK) rc = setup_blocked(g, sms);
   if (rc == GPR_OK && g->max_grid > grid) {  // more CTAs than there are residual partials
     rc = gpr::dalloc(&part, 2 * (size_t)g->max_grid, "cta residuals");
     if (rc == GPR_OK) {
@@ -1340,9 +1347,10 @@ int build_push_layout(gpr_graph *g) {
       g->cta_err = part;
     }
   }
-  if (rc != GPR_OK) {
+  if (rc != GPR_OK) {  // as before the call: the edges go one by one, or a later call builds again
     g->max_grid = grid;
     g->blocked_ok = false;
+    drop_blocked(g);
   }
   g->has_push = rc == GPR_OK;
   return rc;

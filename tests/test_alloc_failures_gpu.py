@@ -1,0 +1,79 @@
+"""What entry points do when one of their device allocations fails: the call falls back
+or reports it, keeps no block that it cannot use, and the next call works.  Each case
+runs in a process of its own with alloc_shim.cc ahead of the library; the failure is a
+status on the host."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+pytestmark = pytest.mark.gpu
+
+PRELUDE = """
+import ctypes, os, sys
+shim = ctypes.CDLL(sys.argv[1], ctypes.RTLD_GLOBAL)
+sys.path[:0] = [sys.argv[2], os.path.join(sys.argv[2], "tests")]
+import numpy as np
+import gardenia_ocl_b200 as G
+import oracle as O
+from graphs import erdos_renyi
+
+def fail(what, status, count=1):
+    shim.shim_fail(what.encode(), status, count)
+
+what, status = sys.argv[3], int(sys.argv[4])
+"""
+
+
+@pytest.fixture(scope="module")
+def shim(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("shim") / "alloc_shim.so")
+    subprocess.run(["/usr/bin/g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-o", out,
+                    os.path.join(ROOT, "tests", "alloc_shim.cc"), "-ldl"], check=True)
+    return out
+
+
+def run(shim, body, what, status):
+    p = subprocess.run([sys.executable, "-c", PRELUDE + body, shim, ROOT, what, str(status)],
+                       capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stdout + p.stderr
+    assert p.stdout.splitlines()[-1] == "done"
+
+
+PUSH = """
+rp, col, od = O.rmat_graph(13, 16, seed=5)
+with G.Graph(rp, col, od, push=True) as g:
+    ref, _ = g.pagerank_push(tol=0.0, max_iter=6)
+before = shim.shim_live()
+g = G.Graph(rp, col, od, push=True)
+made = shim.shim_live()
+fail(what, status)
+if status == G.GPR_ENOMEM:  # edge by edge: sources, destinations and sums are kept, no blocks
+    s, st = g.pagerank_push(tol=0.0, max_iter=6)
+    assert shim.shim_live() == made + 3, (shim.shim_live(), made)
+else:  # reported; nothing kept; the next call builds again
+    try:
+        g.pagerank_push(tol=0.0, max_iter=6)
+        raise SystemExit("no error")
+    except G.GprError as e:
+        assert e.status == status
+    assert shim.shim_live() == made, (shim.shim_live(), made)
+    s, st = g.pagerank_push(tol=0.0, max_iter=6)
+    assert np.array_equal(s, ref)
+assert shim.shim_pending() == 0
+assert st.iterations == 6 and np.abs(s - ref).max() <= 1e-6
+a, _ = g.pagerank(tol=0.0, max_iter=6)
+assert np.abs(a - ref).max() <= 1e-6
+g.close()
+assert shim.shim_live() == before, (shim.shim_live(), before)
+print("done")
+"""
+
+
+@pytest.mark.parametrize("what", ["identity", "largest score", "score sums", "cta residuals"])
+@pytest.mark.parametrize("status", ["GPR_ENOMEM", "GPR_ECUDA"])
+def test_push_layout(G, shim, what, status):
+    run(shim, PUSH, what, getattr(G, status))
