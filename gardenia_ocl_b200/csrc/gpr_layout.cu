@@ -573,7 +573,8 @@ __global__ void k_hot_at(int hot, const int *__restrict__ hot_col, int *hot_at) 
 
 // Columns to stage: the H most frequent ones, H the power of two whose staged
 // gathers, less the 148 H loads that staging costs (one CTA per SM), are most; none
-// unless that is over 1/16 of all entries.  *hot_at: H's index of each column.
+// unless that is over 1/16 of all entries.  *hot_at: H's index of each column, owned by
+// the caller whatever is returned.
 int find_hot_columns(int m, long long nnz, const int *d_Aj, SpmvLayout *L, int **hot_at,
                      cudaStream_t st) {
   Scratch S;
@@ -705,8 +706,18 @@ int build_spmv_layout(int m, long long nnz, const int *d_Ap, const int *d_Aj,
     GPR_TRY(dalloc(&L->slice_at, (size_t)L->n_slices + 1, "slice offsets"));
     k_slice_at<<<grid_for((long long)L->n_slices + 1), 256, 0, st>>>(L->n_slices + 1, L->slice_ptr,
                                                                      L->slice_at);
-    if (hot_columns) GPR_TRY(find_hot_columns(m, nnz, d_Aj, L, &hot_at, st));
-    S.p[4] = hot_at;
+    if (hot_columns) {
+      const int rc = find_hot_columns(m, nnz, d_Aj, L, &hot_at, st);
+      S.p[4] = hot_at;
+      if (rc == GPR_ENOMEM) {  // no room for the search: no staged columns
+        L->hot = 0;
+        dfree(L->hot_col);
+        L->hot_col = nullptr;
+        hot_at = nullptr;
+      } else {
+        GPR_TRY(rc);
+      }
+    }
   }
   GPR_TRY(dalloc(&L->long_col, (size_t)L->long_elems, "long cols"));
   GPR_TRY(dalloc(&L->long_val, (size_t)L->long_elems, "long vals"));

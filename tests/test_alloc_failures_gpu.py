@@ -77,3 +77,49 @@ print("done")
 @pytest.mark.parametrize("status", ["GPR_ENOMEM", "GPR_ECUDA"])
 def test_push_layout(G, shim, what, status):
     run(shim, PUSH, what, getattr(G, status))
+
+
+SPMV = """
+import torch
+rng = np.random.default_rng(3)
+m = 60000
+lens = np.minimum(rng.zipf(1.6, m) - 1, 3000)
+Ap = np.zeros(m + 1, np.int32)
+np.cumsum(lens, out=Ap[1:])
+n = int(Ap[-1])
+Aj = (m * rng.random(n) ** 8).astype(np.int32)  # columns worth staging
+Ax = rng.standard_normal(n).astype(np.float32)
+x = rng.standard_normal(m).astype(np.float32)
+ref = O.spmv_f32(Ap, Aj, Ax, x, np.zeros(m, np.float32))
+absum = np.zeros(m)
+np.add.at(absum, np.repeat(np.arange(m), lens), np.abs(x[Aj] * Ax))
+before = shim.shim_live()
+fail(what, status)
+if status == G.GPR_ENOMEM:
+    A = G.Matrix(Ap, Aj, Ax)
+else:
+    try:
+        G.Matrix(Ap, Aj, Ax)
+        raise SystemExit("no error")
+    except G.GprError as e:
+        assert e.status == status
+    assert shim.shim_live() == before, (shim.shim_live(), before)
+    A = G.Matrix(Ap, Aj, Ax)
+assert shim.shim_pending() == 0
+dx, y = torch.from_numpy(x).cuda(), torch.zeros(m, device="cuda")
+torch.cuda.synchronize()
+A.spmv(dx, y, torch.cuda.current_stream().cuda_stream)
+got = y.cpu().numpy()
+A.close()
+assert shim.shim_live() == before, (shim.shim_live(), before)
+assert np.array_equal(got[lens <= 64], ref[lens <= 64])
+assert np.all(np.abs(got - ref) <= 1e-6 * absum + 1e-30)
+print("done")
+"""
+
+
+@pytest.mark.parametrize("what", ["column counts", "hot columns", "hot column index"])
+@pytest.mark.parametrize("status", ["GPR_ENOMEM", "GPR_ECUDA"])
+def test_spmv_staged_columns(G, shim, what, status):
+    """Without room for the search of columns to stage, the matrix does without."""
+    run(shim, SPMV, what, getattr(G, status))
