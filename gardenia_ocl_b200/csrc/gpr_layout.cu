@@ -688,14 +688,27 @@ int build_spmv_layout(int m, long long nnz, const int *d_Ap, const int *d_Aj,
   const long long short_nnz = std::max(0LL, nnz - long_nnz);
   L->ragged = m <= 0x7fffffff - kSpmvWindow &&
               (L->sell_elems > short_nnz + short_nnz / 8 + 1024 || L->long_elems > nnz / 8);
+  const int windows = (int)ceil_div(m, kSpmvWindow);
+  const size_t slots = (size_t)windows * kSpmvWindow;
   if (L->ragged) {
-    const int windows = (int)ceil_div(m, kSpmvWindow);
-    L->n_slices = windows * (kSpmvWindow / 32);
     row_len = L->sell_len;
     S.p[3] = row_len;
     L->sell_len = nullptr;
-    GPR_TRY(dalloc(&L->sell_len, 32LL * L->n_slices, "slot lengths"));
-    GPR_TRY(dalloc(&L->slot_row, 32LL * L->n_slices, "slot rows"));
+    int rc = dalloc(&L->sell_len, slots, "slot lengths");
+    if (rc == GPR_OK) rc = dalloc(&L->slot_row, slots, "slot rows");
+    if (rc == GPR_OK) rc = dalloc(&L->slice_at, slots / 32 + 1, "slice lines");
+    if (rc == GPR_ENOMEM) {  // no room for the slots: natural order
+      L->ragged = false;
+      for (void *q : {(void *)L->sell_len, (void *)L->slot_row, (void *)L->slice_at}) dfree(q);
+      L->slot_row = L->slice_at = nullptr;
+      L->sell_len = row_len;
+      S.p[3] = nullptr;
+    } else {
+      GPR_TRY(rc);
+    }
+  }
+  if (L->ragged) {
+    L->n_slices = (int)(slots / 32);
     k_spmv_window<<<windows, kSpmvWindow, 0, st>>>(m, row_len, L->slot_row, L->sell_len);
     k_spmv_slice_lens<<<grid_for((long long)L->n_slices + 1), 256, 0, st>>>(
         32 * L->n_slices, L->n_slices, L->sell_len, L->slice_ptr);
@@ -703,7 +716,6 @@ int build_spmv_layout(int m, long long nnz, const int *d_Ap, const int *d_Aj,
     GPR_CUDA(cudaMemcpyAsync(&L->sell_elems, L->slice_ptr + L->n_slices, sizeof(long long),
                              cudaMemcpyDeviceToHost, st));
     GPR_CUDA(cudaStreamSynchronize(st));
-    GPR_TRY(dalloc(&L->slice_at, (size_t)L->n_slices + 1, "slice offsets"));
     k_slice_at<<<grid_for((long long)L->n_slices + 1), 256, 0, st>>>(L->n_slices + 1, L->slice_ptr,
                                                                      L->slice_at);
     if (hot_columns) {

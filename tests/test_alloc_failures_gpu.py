@@ -123,3 +123,10 @@ print("done")
 def test_spmv_staged_columns(G, shim, what, status):
     """Without room for the search of columns to stage, the matrix does without."""
     run(shim, SPMV, what, getattr(G, status))
+
+
+@pytest.mark.parametrize("what", ["slot lengths", "slot rows", "slice lines"])
+@pytest.mark.parametrize("status", ["GPR_ENOMEM", "GPR_ECUDA"])
+def test_spmv_slots(G, shim, what, status):
+    """Without room for sorted rows, a ragged matrix keeps its rows in natural order."""
+    run(shim, SPMV, what, getattr(G, status))
