@@ -371,7 +371,10 @@ int create_impl(int m, long long nnz, const int *any_Ap, const int *any_Aj, cons
   GPR_TRY(rc);
   GPR_TRY(gpr::dalloc(&A->partial, (size_t)A->L.n_chunks, "spmv partials"));
   GPR_TRY(gpr::dalloc(&A->cnt, (size_t)A->L.n_long, "spmv counters"));
-  GPR_CUDA(cudaMemset(A->cnt, 0, sizeof(int) * (A->L.n_long ? A->L.n_long : 1)));
+  GPR_CUDA(cudaMemsetAsync(A->cnt, 0, sizeof(int) * (A->L.n_long ? A->L.n_long : 1), st));
+  // the first multiply may come on a stream that does not wait for this one, and a
+  // recycled block holds another object's data
+  GPR_CUDA(cudaStreamSynchronize(st));
   const long long units = (long long)A->L.n_chunks + A->L.n_slices;
   if (A->L.ragged) {
     int sms = 0;

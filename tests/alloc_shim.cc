@@ -14,6 +14,8 @@ std::mutex mu;
 std::set<void *> live;
 std::string fail_what;
 int fail_status = 0, fail_count = 0;
+std::string call_what;
+void (*call)() = nullptr;
 
 void *real(const char *name) {
   static void *lib = nullptr;
@@ -35,6 +37,7 @@ int dmalloc(void **p, size_t bytes, const char *what) {
   static auto f = reinterpret_cast<int (*)(void **, size_t, const char *)>(
       real("_ZN3gpr7dmallocEPPvmPKc"));
   const int rc = f(p, bytes, what);
+  if (call && call_what == what) call();
   std::lock_guard<std::mutex> lk(mu);
   if (rc == 0) live.insert(*p);
   return rc;
@@ -57,6 +60,11 @@ void shim_fail(const char *what, int status, int count) {
   fail_what = what;
   fail_status = status;
   fail_count = count;
+}
+// `f` is called behind every allocation named `what`.
+void shim_call(const char *what, void (*f)()) {
+  call_what = what;
+  call = f;
 }
 int shim_pending() { return fail_count; }
 int shim_live() { return (int)live.size(); }

@@ -1,7 +1,7 @@
 """What entry points do when one of their device allocations fails: the call falls back
-or reports it, keeps no block that it cannot use, and the next call works.  Each case
-runs in a process of its own with alloc_shim.cc ahead of the library; the failure is a
-status on the host."""
+or reports it, keeps no block that it cannot use, and the next call works; and what
+they owe to a block that held other data.  Each case runs in a process of its own with
+alloc_shim.cc ahead of the library; the failure is a status on the host."""
 import os
 import subprocess
 import sys
@@ -130,3 +130,51 @@ def test_spmv_staged_columns(G, shim, what, status):
 def test_spmv_slots(G, shim, what, status):
     """Without room for sorted rows, a ragged matrix keeps its rows in natural order."""
     run(shim, SPMV, what, getattr(G, status))
+
+
+FIRST_MULTIPLY = """
+import torch
+rng = np.random.default_rng(5)
+m = 20000
+lens = np.full(m, 4)
+lens[:40] = 9000  # three chunks a row
+Ap = np.zeros(m + 1, np.int32)
+np.cumsum(lens, out=Ap[1:])
+n = int(Ap[-1])
+Aj = rng.integers(0, m, n).astype(np.int32)
+Ax = rng.standard_normal(n).astype(np.float32)
+x = rng.standard_normal(m).astype(np.float32)
+ref = O.spmv_f32(Ap, Aj, Ax, x, np.zeros(m, np.float32))
+absum = np.zeros(m)
+np.add.at(absum, np.repeat(np.arange(m), lens), np.abs(x[Aj] * Ax))
+side = torch.cuda.Stream()
+dx = torch.from_numpy(x).cuda()
+ys = [torch.zeros(m, device="cuda") for _ in range(3)]
+ones = np.ones(128, np.int32)
+blocks = [ctypes.c_void_p() for _ in range(4)]
+for p in blocks:
+    assert G.lib().gpr_malloc(ctypes.byref(p), 512) == 0
+    assert G.lib().gpr_memcpy(p, ctypes.c_void_p(ones.ctypes.data), 512) == 0
+torch.cuda.synchronize()
+for p in blocks:
+    G.lib().gpr_free(p)
+# what the default stream does behind the counters' allocation comes late
+late = ctypes.CFUNCTYPE(None)(lambda: torch.cuda._sleep(40000000))
+shim.shim_call(what.encode(), late)
+A = G.Matrix(Ap, Aj, Ax)
+shim.shim_call(b"", ctypes.CFUNCTYPE(None)())
+for y in ys:
+    A.spmv(dx, y, side.cuda_stream)
+side.synchronize()
+torch.cuda.synchronize()
+for y in ys:
+    assert np.all(np.abs(y.cpu().numpy() - ref) <= 1e-6 * absum + 1e-30)
+A.close()
+print("done")
+"""
+
+
+def test_spmv_first_multiply_on_a_stream_of_its_own(G, shim):
+    """The arrival counters are clear before gpr_matrix_create returns: the first
+    multiply on a stream that waits for no other finds them so."""
+    run(shim, FIRST_MULTIPLY, "spmv counters", 0)
