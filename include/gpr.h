@@ -248,7 +248,10 @@ int gpr_pagerank_push(gpr_graph *g, float *any_scores, const gpr_pr_opts *opts,
  * GPR_EINVAL otherwise).  rowptr / col / outdeg are the usual in-CSR and
  * out-degrees over all h_voff[n_graphs] vertices.  h_lopts (n_graphs entries,
  * or NULL for the defaults) gives each graph its own bins: sell_max, chunk,
- * chunk_min as in gpr_graph_create_ex (hot_entries is ignored).  When any
+ * chunk_min as in gpr_graph_create_ex (hot_entries is ignored); the default of
+ * chunk and chunk_min is the larger of what the graph's own edges and the edges
+ * of the batch give, so that in a batch of 2^19 edges and more the last bits of
+ * rows of more than 512 in-edges can differ from the graph solved alone.  When any
  * graph's flags hold GPR_LAYOUT_BLOCKED the batch also builds the blocked
  * form's layout: every graph's rows with in-edges in blocks of block_rows
  * rows that never span two graphs, tiles of up to tile_words words (the

@@ -9,7 +9,7 @@ reproduce the oracle's generator bit for bit.
 import numpy as np
 import pytest
 
-from graphs import erdos_renyi
+from graphs import erdos_renyi, in_csr
 
 pytestmark = pytest.mark.gpu
 
@@ -201,3 +201,28 @@ def test_graph_loop_caps_at_max_iter(G, O, batch):
     assert st1.iterations == 6 and it1.max() == 6
     np.testing.assert_array_equal(s0, s1)
     np.testing.assert_array_equal(it0, it1)
+
+
+def test_default_bins_of_a_batch(G, O):
+    """Default chunks in a batch: the larger of what the graph's own edges (below 2^19:
+    4096) and the batch's edges give.  A graph of a million edges (alone 512) beside
+    as many more has chunks of 512 still, beside twelve million 2048: the bits of
+    a solve with these chunks."""
+    rng = np.random.default_rng(11)
+
+    def graph(m, deg):
+        hubs = [600, 1500, 3000, 5000]
+        src = np.concatenate([rng.choice(m, d, replace=False) for d in hubs]
+                             + [rng.integers(0, m, deg * m)])
+        dst = np.concatenate([np.repeat(np.arange(4), hubs), rng.integers(4, m, deg * m)])
+        return in_csr(m, src, dst)
+
+    big, small = graph(40000, 30), graph(9000, 10)
+    for n_big, chunk in ((2, 512), (10, 2048)):
+        rp, col, od, voff = concat([big] * n_big + [small])
+        with G.MultiGraph(rp, col, od, voff) as mg:
+            s, _, _, _ = mg.pagerank(tol=0.0, max_iter=6)
+        for (g, one), c in (((0, big), chunk), ((n_big, small), 4096)):
+            with G.Graph(*one, chunk=c, chunk_min=c) as alone:
+                ref, _ = alone.pagerank(tol=0.0, max_iter=6)
+            assert np.array_equal(s[voff[g]:voff[g + 1]], ref), (n_big, g)
