@@ -216,7 +216,8 @@ int validate_cols(long long nnz, int ncols, const int *d_col, cudaStream_t st);
 //   even lengths   rows in natural order (x and y locality of a stencil):
 //                  lane l of slice s is row 32 s + l, sell_len[row] its
 //                  length (255: long row, the lane is idle)
-//   ragged         (natural slices would be padded by more than 1/8) rows
+//   ragged         (natural slices would be padded by more than 1/8, or a few long
+//                  chunks would end late: kSpmvWarps) rows
 //                  sorted by descending length inside windows of kSpmvWindow
 //                  rows: slot_row[slot] is the row (-1: none), sell_len[slot]
 //                  its length.  When enough entries fall on few columns, the
@@ -250,6 +251,17 @@ struct SpmvLayout {
 };
 
 constexpr int kSpmvWindow = 1024;  // rows sorted together in a ragged layout
+// Matrices with long rows (over 1/8 of the entries) that are not uneven otherwise take
+// the ragged layout where the chain of loads of one chunk is what k_spmv ends on: the
+// mean chunk is at least a warp's share of all entries (148 SMs x 32 warps) and long
+// enough to take several rounds of k_spmv's 128 entries.  Else k_spmv is faster, whose
+// many light CTAs stream at the memory's rate.  k_spmv_rag / k_spmv, us, rows of k even
+// entries at random columns: 2M entries, k = 130 20.5 / 18.4, 300 18.5 / 14.3, 700 16.4 /
+// 16.4, 1000 16.4 / 18.4, 5000 24.6 / 41.0; 8M, 700 30.7 / 28.7, 1000 28.1 / 24.6, 2000 24.6 /
+// 30.8; 16M, 65 180 / 113, 1000 43 / 41, 5000 61 / 47; 40M, 81 349 / 241.  27-point stencil
+// on 64^3 with 2,000 rows of 1,000: 32.8 / 26.6, with 64 of 30,000: 36.9 / 49.2.
+constexpr int kSpmvWarps = 4736;
+constexpr int kSpmvLongChunk = 640;
 constexpr int kSpmvHotMax = 16384;
 // hot_columns: look for columns to stage in shared memory (a histogram and a sort
 // of the columns; worth it for a matrix that is multiplied more than once).

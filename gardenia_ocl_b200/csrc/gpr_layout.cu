@@ -441,19 +441,24 @@ __global__ void k_spmv_flags(int m, const int *__restrict__ Ap, int sell_max, in
   }
 }
 
+// Padded lengths and chunks of the long rows, and their entries in all.
 __global__ void k_spmv_long_lens(int n_long, const int *__restrict__ rows,
                                  const int *__restrict__ Ap, int chunk, long long *plen,
-                                 int *nch) {
+                                 int *nch, unsigned long long *entries) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned d = 0;
   if (i < n_long) {
     int r = rows[i];
-    long long p = ((long long)(Ap[r + 1] - Ap[r]) + 3) & ~3LL;
+    d = (unsigned)(Ap[r + 1] - Ap[r]);
+    long long p = ((long long)d + 3) & ~3LL;
     plen[i] = p;
     nch[i] = (int)((p + chunk - 1) / chunk);
   } else if (i == n_long) {
     plen[i] = 0;
     nch[i] = 0;
   }
+  d = __reduce_add_sync(0xffffffffu, d);
+  if ((threadIdx.x & 31) == 0 && d) atomicAdd(entries, (unsigned long long)d);
 }
 
 // An entry's stored column: ~h for a hot column (hot_at: h of each column or -1).
@@ -665,8 +670,12 @@ int build_spmv_layout(int m, long long nnz, const int *d_Ap, const int *d_Aj,
   GPR_CUDA(cudaStreamSynchronize(st));
   GPR_TRY(dalloc(&L->long_ptr, (size_t)L->n_long + 1, "long offsets"));
   GPR_TRY(dalloc(&L->row_cbeg, (size_t)L->n_long + 1, "long chunk offsets"));
+  unsigned long long *entries = nullptr, long_nnz = 0;
+  GPR_TRY(dalloc(&entries, 1, "long entries"));
+  S.p[5] = entries;
+  GPR_CUDA(cudaMemsetAsync(entries, 0, sizeof(*entries), st));
   k_spmv_long_lens<<<grid_for((long long)L->n_long + 1), 256, 0, st>>>(
-      L->n_long, L->long_rows, d_Ap, chunk, L->long_ptr, L->row_cbeg);
+      L->n_long, L->long_rows, d_Ap, chunk, L->long_ptr, L->row_cbeg, entries);
   GPR_TRY(exclusive_scan(L->long_ptr, (long long)L->n_long + 1, st));
   GPR_TRY(exclusive_scan(L->row_cbeg, (long long)L->n_long + 1, st));
   // Slices in natural order; ragged when they would be padded by more than 1/8.
@@ -676,7 +685,7 @@ int build_spmv_layout(int m, long long nnz, const int *d_Ap, const int *d_Aj,
   k_spmv_slice_lens<<<grid_for((long long)L->n_slices + 1), 256, 0, st>>>(
       m, L->n_slices, L->sell_len, L->slice_ptr);
   GPR_TRY(exclusive_scan(L->slice_ptr, (long long)L->n_slices + 1, st));
-  long long long_nnz = 0;
+  GPR_CUDA(cudaMemcpyAsync(&long_nnz, entries, sizeof(long_nnz), cudaMemcpyDeviceToHost, st));
   GPR_CUDA(cudaMemcpyAsync(&L->sell_elems, L->slice_ptr + L->n_slices, sizeof(long long),
                            cudaMemcpyDeviceToHost, st));
   GPR_CUDA(cudaMemcpyAsync(&L->long_elems, L->long_ptr + L->n_long, sizeof(long long),
@@ -684,10 +693,12 @@ int build_spmv_layout(int m, long long nnz, const int *d_Ap, const int *d_Aj,
   GPR_CUDA(cudaMemcpyAsync(&L->n_chunks, L->row_cbeg + L->n_long, sizeof(int),
                            cudaMemcpyDeviceToHost, st));
   GPR_CUDA(cudaStreamSynchronize(st));
-  long_nnz = L->long_elems;  // padded to multiples of 4: an upper bound
-  const long long short_nnz = std::max(0LL, nnz - long_nnz);
-  L->ragged = m <= 0x7fffffff - kSpmvWindow &&
-              (L->sell_elems > short_nnz + short_nnz / 8 + 1024 || L->long_elems > nnz / 8);
+  const long long short_nnz = nnz - (long long)long_nnz;
+  const bool uneven = L->sell_elems > short_nnz + short_nnz / 8 + 1024;
+  const bool few_long = L->long_elems > nnz / 8 &&
+                        L->long_elems >= (long long)kSpmvLongChunk * L->n_chunks &&
+                        (double)nnz * L->n_chunks <= (double)kSpmvWarps * L->long_elems;
+  L->ragged = m <= 0x7fffffff - kSpmvWindow && (uneven || few_long);
   const int windows = (int)ceil_div(m, kSpmvWindow);
   const size_t slots = (size_t)windows * kSpmvWindow;
   if (L->ragged) {

@@ -108,3 +108,38 @@ def test_ragged_matrix(G, O, m, hot):
     for out in (got, once):
         assert np.array_equal(out[lens <= 64], ref[lens <= 64])
         assert np.all(np.abs(out - ref) <= 1e-6 * absum + 1e-30)
+
+
+@pytest.mark.parametrize("k,rows,ragged", [(65, 3000, False), (100, 2000, False), (636, 500, False),
+                                           (640, 500, True), (1000, 4736, True),
+                                           (1000, 4737, False), (9000, 40, True)])
+@pytest.mark.parametrize("short", [0, 5000])
+def test_evenly_long_rows(G, O, k, rows, ragged, short):
+    """Rows of k entries each, and `short` rows of 3: natural order unless a chunk (of at
+    most 4096 entries) has 640 entries and a warp's share of all (148 SMs x 32 warps);
+    either way every row is within 1e-6 of its absolute sum of the oracle's."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(k)
+    lens = np.concatenate([np.full(rows, k), np.full(short, 3)])
+    m = len(lens)
+    Ap = np.zeros(m + 1, np.int32)
+    np.cumsum(lens, out=Ap[1:])
+    n = int(Ap[-1])
+    Aj = rng.integers(0, m, n).astype(np.int32)
+    Ax = rng.standard_normal(n).astype(np.float32)
+    x = rng.standard_normal(m).astype(np.float32)
+    y0 = rng.standard_normal(m).astype(np.float32)
+    A = G.Matrix(Ap, Aj, Ax)
+    if short and rows == 4736:  # the short rows' entries take it past the share
+        ragged = False
+    assert A.layout()["n_slices"] == (-(-m // 1024) * 32 if ragged else -(-m // 32))
+    dx, y = torch.from_numpy(x).cuda(), torch.from_numpy(y0.copy()).cuda()
+    torch.cuda.synchronize()
+    A.spmv(dx, y, torch.cuda.current_stream().cuda_stream)
+    got = y.cpu().numpy()
+    A.close()
+    ref = O.spmv_f32(Ap, Aj, Ax, x, y0)
+    absum = np.abs(y0).astype(np.float64)
+    np.add.at(absum, np.repeat(np.arange(m), lens), np.abs(x[Aj] * Ax))
+    assert np.array_equal(got[lens <= 64], ref[lens <= 64])
+    assert np.all(np.abs(got - ref) <= 1e-6 * absum + 1e-30)
