@@ -5,6 +5,7 @@
 #include <dlfcn.h>
 #include <string.h>
 
+#include <map>
 #include <mutex>
 #include <set>
 #include <string>
@@ -12,6 +13,7 @@
 namespace {
 std::mutex mu;
 std::set<void *> live;
+std::map<std::string, size_t> asked;  // bytes of the last allocation of each name
 std::string fail_what;
 int fail_status = 0, fail_count = 0;
 std::string call_what;
@@ -28,6 +30,7 @@ namespace gpr {
 int dmalloc(void **p, size_t bytes, const char *what) {
   {
     std::lock_guard<std::mutex> lk(mu);
+    asked[what] = bytes;
     if (fail_count > 0 && fail_what == what) {
       --fail_count;
       *p = nullptr;
@@ -65,6 +68,11 @@ void shim_fail(const char *what, int status, int count) {
 void shim_call(const char *what, void (*f)()) {
   call_what = what;
   call = f;
+}
+// Bytes of the last allocation named `what` (0: none).
+long long shim_bytes(const char *what) {
+  std::lock_guard<std::mutex> lk(mu);
+  return (long long)asked[what];
 }
 int shim_pending() { return fail_count; }
 int shim_live() { return (int)live.size(); }

@@ -1,6 +1,7 @@
 """What entry points do when one of their device allocations fails: the call falls back
 or reports it, keeps no block that it cannot use, and the next call works; and what
-they owe to a block that held other data.  Each case runs in a process of its own with
+they owe to a block that held other data; and what only the size of an allocation
+shows.  Each case runs in a process of its own with
 alloc_shim.cc ahead of the library; the failure is a status on the host."""
 import os
 import subprocess
@@ -23,6 +24,8 @@ from graphs import erdos_renyi
 
 def fail(what, status, count=1):
     shim.shim_fail(what.encode(), status, count)
+
+shim.shim_bytes.restype = ctypes.c_longlong
 
 what, status = sys.argv[3], int(sys.argv[4])
 """
@@ -178,3 +181,55 @@ def test_spmv_first_multiply_on_a_stream_of_its_own(G, shim):
     """The arrival counters are clear before gpr_matrix_create returns: the first
     multiply on a stream that waits for no other finds them so."""
     run(shim, FIRST_MULTIPLY, "spmv counters", 0)
+
+
+STAGED = """
+import torch
+want, spread = int(what), status  # columns to be staged, and entries beside the limit
+m = 1000000 if want <= 1024 else 300000
+n = 4000000 if want <= 1024 else 8000000
+rng = np.random.default_rng(want + spread)
+lens = np.minimum(rng.zipf(1.5, m), 5000)
+while lens.sum() < n:
+    lens[rng.integers(0, m, 1000)] += 1
+over = int(lens.sum() - n)
+for r in np.argsort(-lens):  # down to n entries in all
+    cut = min(over, int(lens[r]) - 1)
+    lens[r] -= cut
+    over -= cut
+    if not over:
+        break
+Ap = np.zeros(m + 1, np.int32)
+np.cumsum(lens, out=Ap[1:])
+assert Ap[-1] == n
+top = 1024 if want <= 1024 else want
+if want <= 1024:  # exactly the limit (n / 16 and 148 loads a column), and `spread` more
+    hot = n // 16 + 148 * top + spread
+    cols = np.concatenate([np.arange(hot) % top, rng.integers(top, m, n - hot)])
+else:
+    cols = np.concatenate([np.arange(400 * top) % top, rng.integers(top, m, n - 400 * top)])
+Aj = (rng.permutation(m)[rng.permutation(cols)]).astype(np.int32)
+Ax = rng.standard_normal(n).astype(np.float32)
+x = rng.standard_normal(m).astype(np.float32)
+A = G.Matrix(Ap, Aj, Ax)
+assert A.layout()["n_slices"] == -(-m // 1024) * 32  # the ragged layout
+assert shim.shim_bytes(b"hot columns") == 4 * want, shim.shim_bytes(b"hot columns")
+dx, y = torch.from_numpy(x).cuda(), torch.zeros(m, device="cuda")
+torch.cuda.synchronize()
+A.spmv(dx, y, torch.cuda.current_stream().cuda_stream)
+got = y.cpu().numpy()
+A.close()
+ref = O.spmv_f32(Ap, Aj, Ax, x, np.zeros(m, np.float32))
+absum = np.bincount(np.repeat(np.arange(m), lens), np.abs(x[Aj] * Ax), minlength=m)
+assert np.array_equal(got[lens <= 64], ref[lens <= 64])
+assert np.all(np.abs(got - ref) <= 1e-6 * absum + 1e-30)
+print("done")
+"""
+
+
+@pytest.mark.parametrize("want,spread", [(0, 0), (1024, 1), (16384, 0)])
+def test_spmv_columns_are_staged(G, shim, want, spread):
+    """Columns are staged where their entries, less the 148 loads a column, are over 1/16
+    of all: none at the limit, 1024 with an entry more, and as many as fit (16384,
+    64 KB) where that many are frequent; short rows are the oracle's bits."""
+    run(shim, STAGED, str(want), spread)

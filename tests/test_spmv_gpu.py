@@ -78,8 +78,9 @@ def test_empty_matrix(G):
 @pytest.mark.parametrize("hot", [False, True])
 def test_ragged_matrix(G, O, m, hot):
     """Ragged row lengths (windows of 1024 rows sorted by length), a matrix smaller than
-    a window and one row short of and past it, frequent columns staged in shared
-    memory or none frequent; empty rows, lengths around a lane's row (64), a
+    a window and one row short of and past it, columns skewed (at 40,000 rows enough
+    for 1024 of them to be staged; test_spmv_columns_are_staged pins the count) or
+    uniform; empty rows, lengths around a lane's row (64), a
     chunk's round (384) and a chunk (4096).  Short rows are the oracle's bits."""
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(m + hot)
