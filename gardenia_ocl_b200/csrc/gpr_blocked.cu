@@ -188,6 +188,11 @@ unsigned grid_of(long long n, int block = 256) {
 
 }  // namespace
 
+std::mutex &carveout_mutex() {
+  static std::mutex mu;
+  return mu;
+}
+
 void free_blocked_layout(BlockedLayout *B) {
   dfree(B->entry);
   dfree(B->runs);

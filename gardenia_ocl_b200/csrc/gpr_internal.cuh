@@ -7,6 +7,7 @@
 #include <stdio.h>
 
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "gpr.h"
@@ -177,6 +178,11 @@ inline double blocked_bits(int m, long long nnz, double d) {
 }
 
 constexpr int kSumBlocks = 256;  // CTAs of k_sum_abs
+
+// The shared-memory carveout is a preference of a kernel, not of a launch: whoever sets
+// it holds this until the launch (or the occupancy query) that it is for is made, so
+// that handles with other block sizes on other threads do not come between.
+std::mutex &carveout_mutex();
 
 // Rows of the blocked form that stay chunked: the first *row0 rows of the
 // exact-order layout's chunked rows [0, L.n_long), either those with more than

@@ -1097,6 +1097,7 @@ int build_multi(gpr_multigraph *g, const int *h_voff, const int *d_rowptr, const
     GPR_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, g->device));
     g->blocked_ctas = gpr::blocked_ctas_per_sm(B.R > 0 ? B.R : R);
     const int smem = 8 * std::max(B.R, 1);
+    std::unique_lock<std::mutex> carveout(gpr::carveout_mutex());
     for (;;) {
       const void *k = multi_blocked_kernel(g->blocked_ctas);
       cudaFuncAttributes fa;
@@ -1111,6 +1112,7 @@ int build_multi(gpr_multigraph *g, const int *h_voff, const int *d_rowptr, const
       if (per_bsm >= g->blocked_ctas || g->blocked_ctas == 1) break;
       g->blocked_ctas = 1;
     }
+    carveout.unlock();
     g->grid_blocked = sms * g->blocked_ctas;
     g->blocked_ok = g->coop_ok && per_bsm >= g->blocked_ctas;
     g->has_blocked = true;
@@ -1301,7 +1303,7 @@ int solve_phase(gpr_multigraph *g, float *d_scores, const gpr_pr_opts &o, bool b
     }
   } else if (max_cap > 0 && blocked) {
     void *args[] = {&a};
-    // a preference of the function, not of the launch: this batch's
+    std::lock_guard<std::mutex> carveout(gpr::carveout_mutex());
     GPR_CUDA(cudaFuncSetAttribute(multi_blocked_kernel(g->blocked_ctas),
                                   cudaFuncAttributePreferredSharedMemoryCarveout,
                                   g->blocked_carve));

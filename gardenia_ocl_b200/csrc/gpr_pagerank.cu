@@ -764,6 +764,7 @@ int setup_blocked(gpr_graph *g, int sms) {
   // two CTAs and a 28 KB L1).
   g->blocked_ctas = gpr::blocked_ctas_per_sm(g->B.R);
   int per_sm = 0;
+  std::unique_lock<std::mutex> carveout(gpr::carveout_mutex());
   for (;;) {
     // the smallest shared-memory carveout that holds the CTAs: the rest of
     // the SM's 256 KB stays L1
@@ -782,6 +783,7 @@ int setup_blocked(gpr_graph *g, int sms) {
     if (per_sm >= g->blocked_ctas || g->blocked_ctas == 1) break;
     g->blocked_ctas = 1;
   }
+  carveout.unlock();
   g->blocked_ok = g->coop && per_sm >= g->blocked_ctas;
   g->grid_blocked = sms * g->blocked_ctas;
   g->max_grid = std::max(g->max_grid, g->grid_blocked);
@@ -1088,7 +1090,7 @@ int solve_impl(gpr_graph *g, float *d_scores, const gpr_pr_opts &o, int ki, gpr_
   GPR_CUDA(cudaEventRecord(g->e2, st));
   if (o.max_iter > 0 && blocked) {
     void *args[] = {&a};
-    // a preference of the function, not of the launch: this graph's
+    std::lock_guard<std::mutex> carveout(gpr::carveout_mutex());
     GPR_CUDA(cudaFuncSetAttribute(blocked_kernel(g->blocked_ctas),
                                   cudaFuncAttributePreferredSharedMemoryCarveout,
                                   g->blocked_carve));

@@ -291,3 +291,34 @@ def test_auto_keeps_fp32_precision_from_any_start(G, O, kind):
     ref, _, _ = O.pr_f64(rp, col, od, tol=0.0, max_iter=8, init=s0)
     bound = (8 + 4 * np.sqrt(np.diff(rp))) * 2.0 ** -24
     assert np.all(np.abs(s - ref) <= bound * ref)
+
+
+def test_handles_of_different_blocks_on_two_threads(G, O):
+    """The kernel's shared-memory carveout is the one of the graph that is solved,
+    whatever other threads solve: graphs of small and large blocks (two CTAs per SM
+    and one) solved again and again side by side give the bits that they give alone."""
+    import threading
+    graphs = [O.rmat_graph(12, 8, seed=21), O.rmat_graph(15, 8, seed=22)]
+    rows = [256, 12288]
+    kw = dict(tol=0.0, max_iter=4, form=G.FORM_BLOCKED)
+    handles = [G.Graph(*g, blocked=True, block_rows=r) for g, r in zip(graphs, rows)]
+    alone = [h.pagerank(**kw)[0] for h in handles]
+    wrong = []
+
+    def work(i):
+        try:
+            for _ in range(40):
+                s, st = handles[i].pagerank(**kw)
+                if st.iterations != 4 or not np.array_equal(s, alone[i]):
+                    wrong.append(i)
+        except Exception as e:  # a status: the grid was not co-resident
+            wrong.append((i, str(e)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for h in handles:
+        h.close()
+    assert not wrong
