@@ -668,11 +668,10 @@ int build_spmv_layout(int m, long long nnz, const int *d_Ap, const int *d_Aj,
   }
   GPR_CUDA(cudaMemcpyAsync(&L->n_long, nsel, sizeof(int), cudaMemcpyDeviceToHost, st));
   GPR_CUDA(cudaStreamSynchronize(st));
-  GPR_TRY(dalloc(&L->long_ptr, (size_t)L->n_long + 1, "long offsets"));
+  GPR_TRY(dalloc(&L->long_ptr, (size_t)L->n_long + 2, "long offsets"));
   GPR_TRY(dalloc(&L->row_cbeg, (size_t)L->n_long + 1, "long chunk offsets"));
-  unsigned long long *entries = nullptr, long_nnz = 0;
-  GPR_TRY(dalloc(&entries, 1, "long entries"));
-  S.p[5] = entries;
+  // behind the offsets, the long rows' entries without padding
+  unsigned long long *entries = reinterpret_cast<unsigned long long *>(L->long_ptr + L->n_long + 1);
   GPR_CUDA(cudaMemsetAsync(entries, 0, sizeof(*entries), st));
   k_spmv_long_lens<<<grid_for((long long)L->n_long + 1), 256, 0, st>>>(
       L->n_long, L->long_rows, d_Ap, chunk, L->long_ptr, L->row_cbeg, entries);
@@ -685,15 +684,16 @@ int build_spmv_layout(int m, long long nnz, const int *d_Ap, const int *d_Aj,
   k_spmv_slice_lens<<<grid_for((long long)L->n_slices + 1), 256, 0, st>>>(
       m, L->n_slices, L->sell_len, L->slice_ptr);
   GPR_TRY(exclusive_scan(L->slice_ptr, (long long)L->n_slices + 1, st));
-  GPR_CUDA(cudaMemcpyAsync(&long_nnz, entries, sizeof(long_nnz), cudaMemcpyDeviceToHost, st));
   GPR_CUDA(cudaMemcpyAsync(&L->sell_elems, L->slice_ptr + L->n_slices, sizeof(long long),
                            cudaMemcpyDeviceToHost, st));
-  GPR_CUDA(cudaMemcpyAsync(&L->long_elems, L->long_ptr + L->n_long, sizeof(long long),
-                           cudaMemcpyDeviceToHost, st));
+  long long longs[2];  // slots and entries of the long rows
+  GPR_CUDA(cudaMemcpyAsync(longs, L->long_ptr + L->n_long, sizeof(longs), cudaMemcpyDeviceToHost,
+                           st));
   GPR_CUDA(cudaMemcpyAsync(&L->n_chunks, L->row_cbeg + L->n_long, sizeof(int),
                            cudaMemcpyDeviceToHost, st));
   GPR_CUDA(cudaStreamSynchronize(st));
-  const long long short_nnz = nnz - (long long)long_nnz;
+  L->long_elems = longs[0];
+  const long long short_nnz = nnz - longs[1];
   const bool uneven = L->sell_elems > short_nnz + short_nnz / 8 + 1024;
   const bool few_long = L->long_elems > nnz / 8 &&
                         L->long_elems >= (long long)kSpmvLongChunk * L->n_chunks &&

@@ -364,17 +364,19 @@ int create_impl(int m, long long nnz, const int *any_Ap, const int *any_Aj, cons
   if (rc == GPR_OK)
     rc = gpr::build_spmv_layout(m, nnz, (const int *)ap, (const int *)aj, (const float *)ax,
                                 gpr::kSellMaxDefault, gpr::kChunkDefault, hot_columns, &A->L, st);
-  cudaStreamSynchronize(st);
+  if (rc == GPR_OK) rc = gpr::dalloc(&A->partial, (size_t)A->L.n_chunks, "spmv partials");
+  if (rc == GPR_OK) rc = gpr::dalloc(&A->cnt, (size_t)A->L.n_long, "spmv counters");
+  if (rc == GPR_OK)
+    rc = GPR_CUDA_RC(
+        cudaMemsetAsync(A->cnt, 0, sizeof(int) * (A->L.n_long ? A->L.n_long : 1), st));
+  // The counters are clear before the first multiply, which may come on a stream that
+  // does not wait for this one (a recycled block holds another object's data).
+  const cudaError_t se = cudaStreamSynchronize(st);
   if (oap) gpr::dfree(ap);
   if (oaj) gpr::dfree(aj);
   if (oax) gpr::dfree(ax);
   GPR_TRY(rc);
-  GPR_TRY(gpr::dalloc(&A->partial, (size_t)A->L.n_chunks, "spmv partials"));
-  GPR_TRY(gpr::dalloc(&A->cnt, (size_t)A->L.n_long, "spmv counters"));
-  GPR_CUDA(cudaMemsetAsync(A->cnt, 0, sizeof(int) * (A->L.n_long ? A->L.n_long : 1), st));
-  // the first multiply may come on a stream that does not wait for this one, and a
-  // recycled block holds another object's data
-  GPR_CUDA(cudaStreamSynchronize(st));
+  GPR_CUDA(se);
   const long long units = (long long)A->L.n_chunks + A->L.n_slices;
   if (A->L.ragged) {
     int sms = 0;
