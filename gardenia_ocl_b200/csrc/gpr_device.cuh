@@ -194,12 +194,6 @@ __device__ __forceinline__ double block_sum_double(double v) {
   return t;
 }
 
-// Bounded grid barrier of a cooperative launch.  bar[0] counts arrivals,
-// bar[1] is the generation.  When cta_part is given, every CTA first stores
-// its value in cta_part[blockIdx.x] and the last CTA to arrive sums them in
-// CTA order (deterministic) into *sum_out before it opens the next
-// generation.  Waits are bounded by timeout_ns of %globaltimer; on expiry
-// status[0] bit 0 is raised and false is returned.  Call from every thread.
 // Grid barrier without a reduction: `count` (zeroed before the launch) only
 // grows; episode e of a launch (1, 2, ...) is complete when it reaches
 // expect * e, so no CTA has to publish anything after the last arrival and a
@@ -230,6 +224,12 @@ __device__ __forceinline__ bool grid_barrier_count(unsigned *count, unsigned tar
   return s_ok != 0;
 }
 
+// Bounded grid barrier of a cooperative launch.  bar[0] counts arrivals,
+// bar[1] is the generation.  When cta_part is given, every CTA first stores
+// its value in cta_part[blockIdx.x] and the last CTA to arrive sums them in
+// CTA order (deterministic) into *sum_out before it opens the next
+// generation.  Waits are bounded by timeout_ns of %globaltimer; on expiry
+// status[0] bit 0 is raised and false is returned.  Call from every thread.
 __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned expect, double *cta_part,
                                              double cta_value, double *sum_out, int *status,
                                              long long timeout_ns) {

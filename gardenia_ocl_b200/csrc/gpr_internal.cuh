@@ -397,12 +397,15 @@ constexpr int kHotMax = 56832;         // 222 KB: the most one CTA may take
 // share of the edges (148 SMs x 32 warps), so that no warp works on its chunk while
 // the others are done; below 2^19 edges a sweep is a few dependent loads, and the
 // chunks' combination costs more than it saves.  Sweep loop, RMAT, chunks of 512 /
-// 1024 / 2048 / 4096 edges: 10,007 vertices (0.15M edges) 101 / - / - / 91 us, 65,536
-// (0.95M) 236 / 238 / - / 293, 250,007 (3.6M) 678 / 658 / - / 777, 1,000,003 (15M)
-// 2078 / 1751 / 1743 / 1806, 3,000,017 (34M) 4293 / 3821 / 3781 / 3771.  Staging costs
+// 1024 / 2048 / 4096 edges: 10,007 vertices (0.11M edges) 101 / - / - / 91 us, 65,536
+// (0.95M) 236 / 238 / - / 293, 250,007 (3.8M) 678 / 658 / - / 777, 1,000,003 (15M)
+// 2078 / 1751 / 1743 / 1806, 3,000,017 (31M) 4293 / 3821 / 3781 / 3771.  Staging costs
 // every SM the prefix once a sweep: 65,536 vertices with 4096 / 16384 / 32768 staged
 // 208 / 212 / 238 us, 250,007 770 / 729 / 764; 10,007 with 4096 / all staged 168 / 160 us
-// per call.
+// per call.  Other graphs, 20 sweeps, 4096 and 32768 against these defaults: Chung-Lu
+// (exponent 2.1) of 65,536 vertices 275 / 179 us, 250,007 350 / 289, 1,000,003 753 / 765,
+// 2,500,009 1796 / 1801; Erdos-Renyi of 40,000 158 / 162, 65,536 187 / 183, 250,007 402 / 396,
+// 1,000,003 1344 / 1340.
 inline int default_chunk(long long nnz) {
   if (nnz < (1 << 19)) return kChunkDefault;
   int c = 512;

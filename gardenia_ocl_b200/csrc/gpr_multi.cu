@@ -1208,9 +1208,9 @@ int solve_phase(gpr_multigraph *g, float *d_scores, const gpr_pr_opts &o, bool b
     // Where that leaves fewer bits than the largest graph's scores need (a graph whose
     // mass is on few vertices, an earlier solution with its hubs), the batch's whole
     // mass bounds each graph's; without room for the bits the form does not apply.
-    // One exponent for graphs of all sizes costs up to 3 bits from 1/m_g as well (512
-    // graphs of 1,000 to 500,000 vertices: S = 45 against 47.7); those are not searched
-    // for.  A caller who asked for the blocked form by name gets the S of the bound.
+    // One exponent for graphs of all sizes can be short from 1/m_g as well (512 graphs
+    // of 1,000 to 500,000 vertices: S = 47, the largest graph's need 47.5); up to 3 bits
+    // are let pass.  A caller who asked for the blocked form by name gets the S of the bound.
     const double bits_needed = g->fx_bits - log2(1.0 - (double)o.damping);
     if (o.form != GPR_FORM_BLOCKED && (double)S < bits_needed - 3.0) {
       std::vector<double> part(gpr::kSumBlocks);

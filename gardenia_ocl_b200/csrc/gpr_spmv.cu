@@ -36,7 +36,7 @@ constexpr unsigned kFull = 0xffffffffu;
 // 4 / 8 / 16 per round ran at 85% / 99% / 90% of the measured copy bandwidth.
 constexpr int kSpmvU = 8;
 // The same for a ragged layout, and 16-byte loads of columns and of values per lane and
-// round of a chunk: what 64 registers hold.  RMAT, 2,500,009 rows, 38M entries: 8 and
+// round of a chunk: what 64 registers hold.  RMAT, 2,500,009 rows, 31M entries: 8 and
 // 2 189 us, 12 and 3 164 us; two CTAs per SM at 32 registers with 4 and 1 189 us, 768
 // threads with 16 and 4 202 us.
 constexpr int kRagBlock = 1024;
@@ -311,10 +311,11 @@ __device__ __forceinline__ void rag_chunk(const SpArgs &a, const HotX &gx, int c
 // frequent columns is staged in shared memory first; the units (chunks, then slices
 // from wide to narrow) are dealt out to the CTAs and a CTA's warps take them from a
 // counter in shared memory, the next unit's descriptor in flight while they work.
-// RMAT, 2,500,009 rows, 38M entries, y = A x with y cleared: 233 us with rows in
+// RMAT, 2,500,009 rows, 31M entries, y = A x with y cleared: 233 us with rows in
 // natural order (the slices padded, 128 entries of a chunk in flight per warp), 132 us
-// this way (one clock of an SM per 1.0 entries); without staged columns 204 against
-// 189 us (8 entries per round), with 32768 instead of 16384 175 against 164 us.
+// this way (0.6 L2 requests per clock and SM, their path 60% busy); without staged
+// columns 204 against 189 us (8 entries per round), with 32768 instead of 16384 175
+// against 164 us.
 __global__ void __launch_bounds__(kRagBlock, 1) k_spmv_rag(SpArgs a) {
   extern __shared__ float s_x[];
   __shared__ int s_next;
