@@ -94,22 +94,23 @@ std::vector<Block> drain_locked(int device) {
   return out;
 }
 
-// Cached block for a request on device `dev`: the smallest large block that holds
-// `bytes` within 1/8, or the last small block of its class, out of its list.
+// Cached block for a request on device `dev`, out of its list: the smallest large block
+// that holds `bytes` within 1/8 (of equal ones the first in the list, whose free a wait
+// rather covers), or the last small block of its class.
 bool find_locked(size_t bytes, int dev, Block *out) {
-  std::vector<Block> &v = bytes >= kCacheMin ? g_free : g_small[small_class(bytes)];
+  const bool large = bytes >= kCacheMin;
+  std::vector<Block> &v = large ? g_free : g_small[small_class(bytes)];
   int best = -1;
-  for (size_t i = v.size(); i-- > 0;) {
+  for (size_t i = 0; i < v.size(); ++i) {
     const Block &b = v[i];
-    if (b.device != dev || b.bytes < bytes || b.bytes - bytes > bytes / 8) continue;
-    if (best < 0 || b.bytes < v[best].bytes) best = (int)i;
-    if (bytes < kCacheMin) break;
+    if (b.device != dev || (large && (b.bytes < bytes || b.bytes - bytes > bytes / 8))) continue;
+    if (best < 0 || !large || b.bytes < v[best].bytes) best = (int)i;
   }
   if (best < 0) return false;
   *out = v[best];
   v[best] = v.back();
   v.pop_back();
-  (bytes >= kCacheMin ? g_free_bytes : g_small_bytes) -= out->bytes;
+  (large ? g_free_bytes : g_small_bytes) -= out->bytes;
   return true;
 }
 

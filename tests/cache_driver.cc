@@ -95,6 +95,12 @@ void waits() {
   expect(syncs.size() == 1, "a new block waits for nothing");
   device = 0;
   expect(get(1000) == c && syncs.size() == 2, "a block freed since needs a wait of its own");
+  void *x = get(2 << 20), *y = get(2 << 20), *z = get(3000);
+  gpr::dfree(x);
+  gpr::dfree(z);
+  expect(get(3000) == z && syncs.size() == 3, "a wait");
+  gpr::dfree(y);
+  expect(get(2 << 20) == x && syncs.size() == 3, "of equal blocks one that needs no wait");
 }
 
 // A wait that is refused has waited for nothing.
