@@ -182,3 +182,37 @@ def test_push_with_too_small_out_degrees(G, O):
     assert 0 < np.count_nonzero(fin) < m
     assert np.array_equal(fin, np.isfinite(s))
     assert np.abs(s[fin] - ref[fin]).max() <= 1e-6
+
+
+@pytest.mark.parametrize("maker", ["rmat", "er", "star", "ladder"])
+def test_push_edge_by_edge(G, O, maker):
+    """The form without blocks, which one vertex with an edge more than its out-degree
+    says selects: the reference's recurrence with that degree, its stop rule, sweep
+    caps and the bounded wait at its barrier."""
+    rp, col, od = {"rmat": lambda: O.rmat_graph(15, 16, seed=3),
+                   "er": lambda: erdos_renyi(20000, 8, seed=4),
+                   "star": star, "ladder": degree_ladder}[maker]()
+    od = od.copy()
+    some = np.flatnonzero(od > 1)
+    od[some[np.argmin(np.diff(rp)[some])]] -= 1  # of few in-edges: the scores stay bounded
+    tol = 1e-5 if maker in ("star", "ladder") else 1e-6
+    with G.Graph(rp, col, od, push=True) as g:
+        s, st = g.pagerank_push(tol=tol, max_iter=100)
+        t, st_t = g.pagerank_push(tol=0.0, max_iter=5)
+        z, st_z = g.pagerank_push(tol=tol, max_iter=0)
+        o = G.options(tol=tol, max_iter=10, timeout_s=0.5)
+        o.reserved[0] = 1
+        with pytest.raises(G.GprError) as e:
+            g.pagerank_push(opts=o)
+        again, st_a = g.pagerank_push(tol=tol, max_iter=100)
+    assert e.value.status == G.GPR_ETIMEOUT
+    m = len(rp) - 1
+    s0 = np.full(m, np.float32(1.0) / np.float32(m))
+    _, n, _ = O.pr_f64(rp, col, od, tol=tol, max_iter=100)
+    assert abs(st.iterations - n) <= 1 and abs(st_a.iterations - n) <= 1
+    assert st_t.iterations == 5 and st_z.iterations == 0 and np.array_equal(z, s0)
+    for got, sweeps in ((s, st.iterations), (again, st_a.iterations), (t, 5)):
+        ref, off = fp32_sweeps(rp, col, od, s0, sweeps)
+        assert np.all(np.abs(got - ref) <= off), np.max(np.abs(got - ref) / off)
+    # the scores in, all sweeps, the scores out: the blocked solve has one launch more
+    assert st.gpu_launches == 3
