@@ -89,8 +89,10 @@ typedef struct {
  *            28 + log2(edges) for scores of 1/m, fewer the further m x that score
  *            is above 1, 31 or more up to m x score = 2^31), then to FP32.  With a
  *            small S (all scores 1, one vertex that holds all of the mass) scores
- *            of about 1/m keep few correct digits.  Deterministic.  Needs a graph
- *            created with GPR_LAYOUT_BLOCKED and the persistent loop.
+ *            of about 1/m keep few correct digits.  The sums have room for the mass
+ *            of scores whose out-degrees are at least their numbers of edges.
+ *            Deterministic.  Needs a graph created with GPR_LAYOUT_BLOCKED and the
+ *            persistent loop.
  *   AUTO     BLOCKED when the graph has its layout, at least 50,331,648 edges
  *            (below that EXACT measured faster: RMAT scale 21 3.6 vs 3.9 ms,
  *            scale 22 7.6 vs 6.8 ms) and the persistent loop runs, else EXACT.
